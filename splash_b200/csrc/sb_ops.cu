@@ -3,8 +3,11 @@
 // Each replaces the reference operator named at its entry point in include/splash_b200.h.
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "sb_dequant.cuh"
 #include "sb_dot.cuh"
+#include "sb_select.cuh"
 
 namespace sb {
 
@@ -318,183 +321,31 @@ __global__ void kv_path_commit_kernel(SbKvLayer c, const uint32_t *page_table, u
   }
 }
 
-// ---- selection: one block of 1024 threads per row ----
-constexpr uint32_t kSentinel = 0xFFFFFFFFu;
-constexpr uint32_t kShard = 256;
-constexpr uint32_t kDrawCandidates = 16, kNoDraw = 0xff;  // a row's draft candidates; "no child drawn" (runtime/metal/abi/ExecutionGeometry.h:63)
+// ---- selection: a cluster of eight CTAs a row (sb_select.cuh) ----
+// The view of lane z: its rows are rows 16 z .. of every row-indexed buffer, its uniforms the 80 from 80 z on, its policy its own.
+__device__ __forceinline__ SbSampleArgs lane_selection(SbSampleArgs a, uint32_t z) {
+  const uint32_t r0 = kLaneRows * z;
+  a.logits += size_t(r0) * a.logit_stride, a.input_tokens += r0, a.selected += r0;
+  if (a.uniforms) a.uniforms += 80 * z;
+  if (a.workspace) a.workspace += size_t(r0) * (2 * ((a.vocab + kShard - 1) / kShard) + 8);
+  if (a.cut_out) a.cut_out += 2 * r0;
+  if (a.candidate_ids) a.candidate_ids += kDrawCandidates * r0, a.candidate_q += kDrawCandidates * r0, a.draws += 4 * r0;
+  if (a.lane_policies) {
+    const SbLanePolicy q = a.lane_policies[z];
+    a.temperature = q.temperature, a.min_p = q.min_p, a.top_k = q.top_k, a.top_p = q.top_p;
+  }
+  return a;
+}
+
 constexpr int kSampleThreads = 1024;
-
-__device__ __forceinline__ bool selectable(float x) { return !(isnan(x) || x == -INFINITY); }
-
-// ---- the end of a row's distribution: min-p, then top-k, then the top-p nucleus (sampling.metal:604-668) ----
-// A token stays iff its key (order-preserving bits of its logit, -0 as +0) is above cut.key, or equal to it with an id
-// up to cut.id. Every search walks the 32 key bits from the top with one block-wide measurement per bit; masses are the
-// shard sums (256 ids in id order) added in shard order by one thread, as everywhere in this kernel.
-constexpr uint32_t kMaxFilterShards = 1024;  // vocabulary up to 262144 with filters
-struct RowCut {
-  uint32_t key, id;
-};
-__device__ __forceinline__ uint32_t logit_key(float x) {
-  if (x == 0.0f) x = 0.0f;
-  const uint32_t u = __float_as_uint(x);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float key_logit(uint32_t key) {
-  return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
-}
-__device__ __forceinline__ bool cut_keeps(const RowCut c, float x, uint32_t v) {
-  if (!selectable(x)) return false;
-  const uint32_t k = logit_key(x);
-  return k > c.key || (k == c.key && v <= c.id);
-}
-struct FilterScratch {
-  float shard_mass[kMaxFilterShards];
-  uint32_t counts[kSampleThreads];
-  uint32_t warp_counts[32];
-  uint32_t count, pick_thread, pick_rank, id;
-  float mass;
-};
-// Count and mass of the kept tokens whose key is at least `key` (above it when `strict`); every thread gets both.
-__device__ void block_measure(const float *l, uint32_t vocab, RowCut cut, uint32_t key, bool strict, bool want_mass, float mx, float inv_t,
-                              FilterScratch &fs, uint32_t &count, float &mass) {
-  const uint32_t tid = threadIdx.x, shards = (vocab + kShard - 1) / kShard;
-  uint32_t mine = 0;
-  for (uint32_t s = tid; s < shards; s += kSampleThreads) {
-    float sum = 0.0f;
-    const uint32_t end = min(vocab, (s + 1) * kShard);
-    for (uint32_t v = s * kShard; v < end; ++v) {
-      const float x = l[v];
-      if (!cut_keeps(cut, x, v)) continue;
-      const uint32_t k = logit_key(x);
-      if (strict ? k > key : k >= key) {
-        ++mine;
-        if (want_mass) sum = __fadd_rn(sum, expf(__fmul_rn(__fsub_rn(x, mx), inv_t)));
-      }
-    }
-    fs.shard_mass[s] = sum;
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-  if ((tid & 31) == 0) fs.warp_counts[tid >> 5] = mine;
-  __syncthreads();
-  if (tid == 0) {
-    uint32_t c = 0;
-    for (int w = 0; w < kSampleThreads / 32; ++w) c += fs.warp_counts[w];
-    float m = 0.0f;
-    if (want_mass)
-      for (uint32_t s = 0; s < shards; ++s) m = __fadd_rn(m, fs.shard_mass[s]);
-    fs.count = c, fs.mass = m;
-  }
-  __syncthreads();
-  count = fs.count, mass = fs.mass;
-  __syncthreads();
-}
-// The id of the n-th (1-based) kept token whose key equals `key`, in id order.
-__device__ uint32_t block_nth_tie(const float *l, uint32_t vocab, RowCut cut, uint32_t key, uint32_t n, FilterScratch &fs) {
-  const uint32_t tid = threadIdx.x, chunk = (vocab + kSampleThreads - 1) / kSampleThreads;
-  const uint32_t v0 = min(vocab, tid * chunk), v1 = min(vocab, v0 + chunk);
-  uint32_t mine = 0;
-  for (uint32_t v = v0; v < v1; ++v) mine += cut_keeps(cut, l[v], v) && logit_key(l[v]) == key;
-  fs.counts[tid] = mine;
-  if (tid == 0) fs.id = kSentinel;
-  __syncthreads();
-  if (tid == 0) {
-    uint32_t before = 0, t = 0;
-    for (; t < kSampleThreads && before + fs.counts[t] < n; ++t) before += fs.counts[t];
-    fs.pick_thread = t, fs.pick_rank = n - before;
-  }
-  __syncthreads();
-  if (tid == fs.pick_thread) {
-    uint32_t rank = fs.pick_rank;
-    for (uint32_t v = v0; v < v1; ++v)
-      if (cut_keeps(cut, l[v], v) && logit_key(l[v]) == key && --rank == 0) {
-        fs.id = v;
-        break;
-      }
-  }
-  __syncthreads();
-  const uint32_t id = fs.id;
-  __syncthreads();
-  return id;
-}
-__device__ RowCut distribution_end(const float *l, uint32_t vocab, float mx, float temperature, float inv_t, float min_p, uint32_t top_k,
-                                   float top_p, FilterScratch &fs) {
-  RowCut cut{0u, kSentinel};
-  uint32_t kept_count, count;
-  float kept_mass, mass;
-  block_measure(l, vocab, cut, 0u, false, true, mx, inv_t, fs, kept_count, kept_mass);
-  if (min_p > 0.0f) {
-    const float t = fminf(__fadd_rn(mx, __fmul_rn(temperature, logf(min_p))), mx);
-    block_measure(l, vocab, cut, logit_key(t), false, true, mx, inv_t, fs, count, mass);
-    if (count < kept_count) cut = RowCut{logit_key(t), kSentinel}, kept_count = count, kept_mass = mass;
-  }
-  if (top_k > 0 && top_k < kept_count) {
-    uint32_t key = 0;  // the largest key with at least top_k kept tokens at or above it
-    for (int bit = 31; bit >= 0; --bit) {
-      const uint32_t cand = key | (1u << bit);
-      block_measure(l, vocab, cut, cand, false, false, mx, inv_t, fs, count, mass);
-      if (count >= top_k) key = cand;
-    }
-    block_measure(l, vocab, cut, key, true, true, mx, inv_t, fs, count, mass);
-    const uint32_t need = top_k - count;
-    const uint32_t id = block_nth_tie(l, vocab, cut, key, need, fs);
-    cut = RowCut{key, id};
-    kept_count = top_k;
-    kept_mass = __fadd_rn(mass, __fmul_rn(float(need), expf(__fmul_rn(__fsub_rn(key_logit(key), mx), inv_t))));
-  }
-  if (top_p > 0.0f && top_p < 1.0f) {
-    const float nucleus = __fmul_rn(top_p, kept_mass);
-    uint32_t key = 0;  // the largest key whose kept tokens at or above it weigh more than the nucleus
-    bool found = false;
-    for (int bit = 31; bit >= 0; --bit) {
-      const uint32_t cand = key | (1u << bit);
-      block_measure(l, vocab, cut, cand, false, true, mx, inv_t, fs, count, mass);
-      if (mass > nucleus) key = cand, found = true;
-    }
-    if (!found) {
-      block_measure(l, vocab, cut, 0u, false, true, mx, inv_t, fs, count, mass);
-      found = mass > nucleus;
-    }
-    if (found) {  // rounding may leave the nucleus unreached: then everything kept so far stays
-      uint32_t above_count, at_count;
-      float above_mass, at_mass;
-      block_measure(l, vocab, cut, key, true, true, mx, inv_t, fs, above_count, above_mass);
-      block_measure(l, vocab, cut, key, false, false, mx, inv_t, fs, at_count, at_mass);
-      const uint32_t ties = at_count - above_count;
-      if (ties > 0) {
-        const float w = expf(__fmul_rn(__fsub_rn(key_logit(key), mx), inv_t));
-        const float q = fminf(fmaxf(__fdiv_rn(__fsub_rn(nucleus, above_mass), w), 0.0f), float(ties - 1));
-        const uint32_t keep = 1u + uint32_t(q);
-        const uint32_t id = block_nth_tie(l, vocab, cut, key, keep, fs);
-        cut = RowCut{key, id};
-      }
-    }
-  }
-  return cut;
-}
-
-// One row's selection by one block (row blockIdx.x of lane blockIdx.y).
-__device__ __forceinline__ void sample_row(const SbSampleArgs &a_in) {
-  __shared__ FilterScratch fs;
+// One row's selection by one block: many greedy rows, and vocabularies above kSelectVocab (which take no filters); row r of the
+// lane's view a.
+__device__ __forceinline__ void sample_row(const SbSampleArgs &a, uint32_t r) {
   __shared__ float best_v[32];
   __shared__ uint32_t best_i[32];
   __shared__ float s_max;
   __shared__ uint32_t s_top;
-  // Lanes (blockIdx.y): lane z's rows are rows 16 z .. of every row-indexed buffer, its uniforms the 80 from 80 z on.
-  SbSampleArgs a = a_in;
-  {
-    const uint32_t z = blockIdx.y, r0 = kLaneRows * z;
-    a.logits += size_t(r0) * a.logit_stride, a.input_tokens += r0, a.selected += r0;
-    if (a.uniforms) a.uniforms += 80 * z;
-    if (a.workspace) a.workspace += size_t(r0) * (2 * ((a.vocab + kShard - 1) / kShard) + 8);
-    if (a.cut_out) a.cut_out += 2 * r0;
-    if (a.candidate_ids) a.candidate_ids += kDrawCandidates * r0, a.candidate_q += kDrawCandidates * r0, a.draws += 4 * r0;
-    if (a.lane_policies) {  // the lane's own policy
-      const SbLanePolicy q = a.lane_policies[z];
-      a.temperature = q.temperature, a.min_p = q.min_p, a.top_k = q.top_k, a.top_p = q.top_p;
-    }
-  }
-  const uint32_t r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float *l = a.logits + size_t(r) * a.logit_stride;
   // Greedy: value descending, id ascending.
   float bv = -INFINITY;
@@ -503,16 +354,11 @@ __device__ __forceinline__ void sample_row(const SbSampleArgs &a_in) {
     const float x = l[v];
     if (selectable(x) && (bi == kSentinel || x > bv)) bv = x, bi = v;
   }
-  auto better = [](float v1, uint32_t i1, float v2, uint32_t i2) {
-    if (i2 == kSentinel) return true;
-    if (i1 == kSentinel) return false;
-    return v1 > v2 || (v1 == v2 && i1 < i2);
-  };
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
     const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (!better(bv, bi, ov, oi)) bv = ov, bi = oi;
+    if (!better_token(bv, bi, ov, oi)) bv = ov, bi = oi;
   }
   if (lane == 0) best_v[warp] = bv, best_i[warp] = bi;
   __syncthreads();
@@ -520,7 +366,7 @@ __device__ __forceinline__ void sample_row(const SbSampleArgs &a_in) {
     float v = best_v[0];
     uint32_t i = best_i[0];
     for (int w = 1; w < kSampleThreads / 32; ++w)
-      if (!better(v, i, best_v[w], best_i[w])) v = best_v[w], i = best_i[w];
+      if (!better_token(v, i, best_v[w], best_i[w])) v = best_v[w], i = best_i[w];
     s_max = v, s_top = i;
   }
   __syncthreads();
@@ -535,13 +381,10 @@ __device__ __forceinline__ void sample_row(const SbSampleArgs &a_in) {
   float *shard = a.workspace + size_t(r) * (2 * shards + 8), *shard2 = shard + shards;
   const bool has_child = !a.candidate_ids && r + 1 < a.rows;  // (with the draft's candidates given, the children are the rows' draws)
   const uint32_t child = has_child ? a.input_tokens[r + 1] : kSentinel;
-  RowCut cut{0u, kSentinel};
-  if (a.min_p > 0.0f || (a.top_k > 0 && a.top_k < a.vocab) || (a.top_p > 0.0f && a.top_p < 1.0f))
-    cut = distribution_end(l, a.vocab, mx, a.temperature, inv_t, a.min_p, a.top_k, a.top_p, fs);
-  if (a.cut_out && tid == 0) a.cut_out[2 * r] = cut.key, a.cut_out[2 * r + 1] = cut.id;
+  if (a.cut_out && tid == 0) a.cut_out[2 * r] = 0u, a.cut_out[2 * r + 1] = kSentinel;  // (everything selectable stays)
   auto weight = [&](uint32_t v) {
     const float x = l[v];
-    return cut_keeps(cut, x, v) ? expf(__fmul_rn(__fsub_rn(x, mx), inv_t)) : 0.0f;
+    return selectable(x) ? expf(__fmul_rn(__fsub_rn(x, mx), inv_t)) : 0.0f;
   };
   for (uint32_t s = tid; s < shards; s += kSampleThreads) {
     float sum = 0.0f, sum2 = 0.0f;
@@ -683,10 +526,17 @@ __device__ __forceinline__ void sample_row(const SbSampleArgs &a_in) {
   a.selected[r] = pick;
 }
 
-__global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SbSampleArgs a) {
+// grid (8 rows, lanes), a cluster a row; `cluster` false: grid (rows, lanes), a block a row.
+template <bool CLUSTER> __global__ void __launch_bounds__(CLUSTER ? kSelectThreads : kSampleThreads, CLUSTER ? 2 : 1) sample_kernel(const SbSampleArgs a) {
+  extern __shared__ __align__(16) uint8_t select_smem[];
   pdl_launch_dependents();
   pdl_wait();
-  sample_row(a);
+  if (CLUSTER) {
+    SelectRow::sync();  // every CTA of the row runs before any writes into it
+    select_row(lane_selection(a, blockIdx.y), blockIdx.x / kSelectCtas, select_smem);
+  } else {
+    sample_row(lane_selection(a, blockIdx.y), blockIdx.x);
+  }
 }
 
 // ---- acceptance: one thread ----
@@ -747,20 +597,27 @@ __device__ __forceinline__ void commit_lane(const SbSelectAcceptArgs &c, uint32_
   }
 }
 
-// Selection, acceptance and the lane's commit in one launch: a block per row selects (sample_row), and the block of a
-// lane that finishes last (a ticket per lane, drawn after the block's selection is visible) walks the accepted path
+// Selection, acceptance and the lane's commit in one launch: a cluster (or block) per row selects, and the one of a
+// lane that finishes last (a ticket per lane, drawn after the row's selection is visible) walks the accepted path
 // and commits the lane. The ticket word returns to zero for the next launch.
-__global__ void __launch_bounds__(kSampleThreads) select_accept_kernel(const SbSelectAcceptArgs c_in) {
+template <bool CLUSTER> __global__ void __launch_bounds__(CLUSTER ? kSelectThreads : kSampleThreads, CLUSTER ? 2 : 1) select_accept_kernel(const SbSelectAcceptArgs c_in) {
+  extern __shared__ __align__(16) uint8_t select_smem[];
   pdl_launch_dependents();
   pdl_wait();
-  const uint32_t lane = blockIdx.y;
+  const uint32_t lane = blockIdx.y, row = CLUSTER ? blockIdx.x / kSelectCtas : blockIdx.x;
   // The lane's own rows (blocks of different lengths step together): the blocks of the slots past them select nothing.
   const uint32_t lane_rows = c_in.lane_rows ? min(c_in.lane_rows[lane], c_in.sample.rows) : c_in.sample.rows;
-  if (blockIdx.x < lane_rows) {
-    SbSampleArgs s = c_in.sample;
+  if (row < lane_rows) {
+    SbSampleArgs s = lane_selection(c_in.sample, lane);
     s.rows = lane_rows;
-    sample_row(s);
+    if (CLUSTER) {
+      SelectRow::sync();  // every CTA of the row runs before any writes into it
+      select_row(s, row, select_smem);
+    } else {
+      sample_row(s, row);
+    }
   }
+  if (CLUSTER && blockIdx.x % kSelectCtas) return;
   if (threadIdx.x != 0) return;
   __threadfence();
   if (atomicAdd(c_in.tickets + lane, 1u) != c_in.sample.rows - 1) return;
@@ -889,6 +746,39 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const SbMoeRouteArgs a) 
     a.weights[size_t(row) * routes + lane] = a.sigmoid_normalized ? (1.0f / (1.0f + exp2f(-1.44269504089f * ordered[lane]))) / (den + 1e-20f)
                                                                    : exp2f((ordered[lane] - ordered[0]) * 1.44269504089f) / den;
   }
+}
+
+// A selection over rows x lanes: the cluster kernel up to its vocabulary (a greedy launch keeps no logits in shared memory), the
+// block kernel above. A greedy row is one short pass, and what counts is how many rows run at once: 37 clusters are resident
+// (two CTAs a SM), so up to 32 greedy rows take clusters (16 rows of 151,936: 15.1 us against 20.8 with a block a row) and more
+// take a block each, all resident together (128 rows: 29.6 us against 38.4; 512 rows: 92 against 133). Sampled rows are the
+// other way round (128 rows without filters: 122 us against 182; 512 rows: 423 against 548) until the vocabulary leaves room
+// for one CTA a SM only (above some 160,000 ids): without filters 128 rows of 232,001 take 220 us against 259, 512 rows 804
+// against 800, so from 256 such rows on a row is a block's; with filters clusters win at every count (512 rows: 2.1 ms
+// against 34.6).
+constexpr uint32_t kGreedyClusterRows = 32, kPlainClusterRows = 256;
+constexpr size_t kTwoCtasSmem = 113 * 1024;
+template <class A> static int launch_selection(void (*cluster)(A), void (*block)(A), const SbSampleArgs &s, cudaStream_t stream, const A &args) {
+  const bool staged = s.lane_policies || (s.temperature != 0.0f && s.uniforms);
+  const uint32_t rows = s.rows * std::max(1u, s.lanes);
+  const bool filtered = s.lane_policies || s.min_p > 0.0f || (s.top_k > 0 && s.top_k < s.vocab) || (s.top_p > 0.0f && s.top_p < 1.0f);
+  const bool clusters = s.vocab <= kSelectVocab && (!staged ? rows <= kGreedyClusterRows
+                                                            : filtered || rows < kPlainClusterRows || select_smem_bytes(s.vocab) <= kTwoCtasSmem);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(clusters ? s.rows * kSelectCtas : s.rows, std::max(1u, s.lanes));
+  cfg.blockDim = dim3(clusters ? kSelectThreads : kSampleThreads);
+  cfg.dynamicSmemBytes = !clusters ? 0 : staged ? select_smem_bytes(s.vocab) : (sizeof(SelectShared) + 15) / 16 * 16;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = ctx().pdl ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = kSelectCtas, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = clusters ? 2 : 1;
+  if (clusters) SB_CUDA(cudaFuncSetAttribute(cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, int(select_smem_bytes(kSelectVocab))));
+  SB_CUDA(cudaLaunchKernelEx(&cfg, clusters ? cluster : block, args));
+  return SB_OK;
 }
 
 template <class... Args>
@@ -1023,11 +913,11 @@ int sb_sample_verify(void *stream, const SbSampleArgs *a) {
   SB_REQUIRE(a->temperature == 0.0f || (a->uniforms && a->workspace), "sb_sample_verify: a sampled policy needs uniforms and a workspace");
   SB_REQUIRE(a->min_p >= 0.0f && a->min_p <= 1.0f && a->top_p >= 0.0f, "sb_sample_verify: min_p %g outside 0..1 or negative top_p", double(a->min_p));
   const bool filtered = a->min_p > 0.0f || (a->top_k > 0 && a->top_k < a->vocab) || (a->top_p > 0.0f && a->top_p < 1.0f);
-  SB_REQUIRE(!filtered || a->vocab <= kMaxFilterShards * kShard, "sb_sample_verify: min-p / top-k / top-p support vocabularies up to %u", kMaxFilterShards * kShard);
+  SB_REQUIRE(!filtered || a->vocab <= kSelectVocab, "sb_sample_verify: min-p / top-k / top-p support vocabularies up to %u", kSelectVocab);
   SB_REQUIRE(!a->candidate_ids || (a->candidate_q && a->draws), "sb_sample_verify: candidates come with their draft probabilities and the rows' draws");
   SB_REQUIRE(a->lanes <= 64, "sb_sample_verify: %u lanes (up to 64)", a->lanes);
-  SB_REQUIRE(!a->lane_policies || (a->uniforms && a->workspace && a->vocab <= kMaxFilterShards * kShard), "sb_sample_verify: policies a lane need uniforms, the workspace and a vocabulary the filters take");
-  return launch(sample_kernel, dim3(a->rows, std::max(1u, a->lanes)), dim3(kSampleThreads), as_stream(stream), *a);
+  SB_REQUIRE(!a->lane_policies || (a->uniforms && a->workspace && a->vocab <= kSelectVocab), "sb_sample_verify: policies a lane need uniforms, the workspace and a vocabulary the filters take");
+  return launch_selection(sample_kernel<true>, sample_kernel<false>, *a, as_stream(stream), *a);
 }
 
 int sb_sample_admit(void *stream, const SbAdmitArgs *a) {
@@ -1070,16 +960,16 @@ int sb_select_accept(void *stream, const SbSelectAcceptArgs *c) {
   SB_REQUIRE(a->temperature == 0.0f || (a->uniforms && a->workspace), "sb_select_accept: a sampled policy needs uniforms and a workspace");
   SB_REQUIRE(a->min_p >= 0.0f && a->min_p <= 1.0f && a->top_p >= 0.0f, "sb_select_accept: min_p %g outside 0..1 or negative top_p", double(a->min_p));
   const bool filtered = a->min_p > 0.0f || (a->top_k > 0 && a->top_k < a->vocab) || (a->top_p > 0.0f && a->top_p < 1.0f);
-  SB_REQUIRE(!filtered || a->vocab <= kMaxFilterShards * kShard, "sb_select_accept: min-p / top-k / top-p support vocabularies up to %u", kMaxFilterShards * kShard);
+  SB_REQUIRE(!filtered || a->vocab <= kSelectVocab, "sb_select_accept: min-p / top-k / top-p support vocabularies up to %u", kSelectVocab);
   SB_REQUIRE(!a->candidate_ids || (a->candidate_q && a->draws), "sb_select_accept: candidates come with their draft probabilities and the rows' draws");
   SB_REQUIRE(a->lanes <= 64, "sb_select_accept: %u lanes (up to 64)", a->lanes);
-  SB_REQUIRE(!a->lane_policies || (a->uniforms && a->workspace && a->vocab <= kMaxFilterShards * kShard), "sb_select_accept: policies a lane need uniforms, the workspace and a vocabulary the filters take");
+  SB_REQUIRE(!a->lane_policies || (a->uniforms && a->workspace && a->vocab <= kSelectVocab), "sb_select_accept: policies a lane need uniforms, the workspace and a vocabulary the filters take");
   SB_REQUIRE(b->input_tokens == a->input_tokens && b->tokens == a->selected && b->tree && b->results, "sb_select_accept: acceptance reads the selection's rows: same input tokens, tokens = selected");
   SB_REQUIRE(b->rows == a->rows && b->remaining >= 1 && std::max(1u, b->lanes) == std::max(1u, a->lanes), "sb_select_accept: selection and acceptance disagree on rows or lanes");
   SB_REQUIRE(b->n_stop == 0 || b->stop_tokens, "sb_select_accept: stop tokens missing");
   SB_REQUIRE(!c->committed || (c->pending_rows && c->pending_path), "sb_select_accept: the commit needs the lanes' pending words");
   SB_REQUIRE((c->advance & 0xffu) <= 3 && ((c->advance & 0xffu) != 3 || c->advance >> 8 == a->rows), "sb_select_accept: advance = 0x%x", c->advance);
-  return launch(select_accept_kernel, dim3(a->rows, std::max(1u, a->lanes)), dim3(kSampleThreads), as_stream(stream), *c);
+  return launch_selection(select_accept_kernel<true>, select_accept_kernel<false>, *a, as_stream(stream), *c);
 }
 
 int sb_accept(void *stream, const SbAcceptArgs *a) {

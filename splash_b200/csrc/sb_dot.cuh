@@ -12,9 +12,9 @@ namespace sb {
 
 constexpr int kDotGroups = 8;
 
-// acc[a][b] = group `group`'s partial sum of x[a] . w[b] (all lanes hold it).
+// acc[a][b] = this lane's share of group `group`'s partial sum of x[a] . w[b].
 template <int NW, int NX>
-__device__ __forceinline__ void warp_dot_group_f32_bf16(const float *const (&w)[NW], const uint16_t *const (&x)[NX], uint32_t k, uint32_t lane,
+__device__ __forceinline__ void lane_dot_group_f32_bf16(const float *const (&w)[NW], const uint16_t *const (&x)[NX], uint32_t k, uint32_t lane,
                                                         uint32_t group, float (&acc)[NX][NW]) {
 #pragma unroll
   for (int a = 0; a < NX; ++a)
@@ -42,6 +42,13 @@ __device__ __forceinline__ void warp_dot_group_f32_bf16(const float *const (&w)[
       }
     }
   }
+}
+
+// The same summed over the lanes (all of them hold it).
+template <int NW, int NX>
+__device__ __forceinline__ void warp_dot_group_f32_bf16(const float *const (&w)[NW], const uint16_t *const (&x)[NX], uint32_t k, uint32_t lane,
+                                                        uint32_t group, float (&acc)[NX][NW]) {
+  lane_dot_group_f32_bf16<NW, NX>(w, x, k, lane, group, acc);
 #pragma unroll
   for (int a = 0; a < NX; ++a)
 #pragma unroll

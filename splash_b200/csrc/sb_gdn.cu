@@ -1,24 +1,38 @@
-// Gated-DeltaNet verify step of one lane and one layer with fp32 state and warp-shuffle reductions.
+// Gated-DeltaNet verify step of one lane and one layer with fp32 state.
 //
 // Takes the place of the reference's verify_gdn_fused* kernels (runtime/metal/kernels/decode/gdn.metal:
 // prologue :139-264, fold :270-298, chain scan :312-415, gate :489-526; primitives
 // runtime/metal/kernels/common/gdn_primitives.h:63-106) and of ops::GDN::addDecode / addFold
 // (runtime/ops/GDN.cpp:225-328).
 //
-//   grid     (4, value_heads): the reference runs one threadgroup per value head (48 on the 27B shape,
+//   grid     (4, value_heads, lanes): the reference runs one threadgroup per value head (48 on the 27B shape,
 //            too few for 148 SMs); a head's 128 state rows (value dimensions) are independent given
-//            k, v and the gates, so each CTA takes 32 of them
-//   CTA      256 threads; warp w owns state rows 4w..4w+3 of the CTA's 32, each lane four fp32 key
-//            columns of each row (16 registers of state); dot products are butterfly shuffles
+//            k, v and the gates, so each CTA takes 32 of them; a head's four CTAs are a cluster and divide what the
+//            head's rows share (gate projection, q / k convolution and norms, the rows' inner products, the output norm)
 //   steps    (1) conv history = last three input rows before the block (carried rows ++ pending rows);
 //            (2) conv + SiLU, q/k RMS norm and scales (2^-7, 128^-1/2), beta and decay per row;
-//            (3) fold the pending rows into the state -> committed state stored; (4) chain scan from the
-//            committed state, outputs only; (5) the head's last CTA normalises (RMS over the 128 value
-//            dimensions), gates by silu(z) and writes the hidden rows; (6) this step's tape
+//            (3) fold the pending rows into the state -> committed state stored; (4) the rows' outputs from the
+//            committed state; (5) RMS norm over the 128 value dimensions, gate by silu(z), the hidden rows; (6) this step's tape
+//
+// The delta rule without its serial chain. A row's step S' = d S + u k^T, u = beta (v - d S k) touches the whole state, and 22
+// of them (6 folded, 16 scanned) one after the other, each a reduction across lanes, took most of the kernel (23.4 us a call
+// of one lane, 106 us of eight, where moving the state takes 1 and 8). The state after the block is never stored, so it is
+// never formed: with S the committed state, P(t) a row's path from the anchor and G(t, j) the product of the decays on it
+// after row j (D_t: of all of them),
+//   u_t = beta_t (v_t - D_t (S k_t) - sum over j in P(t), j != t, of G(t, j) (k_j . k_t) u_j)
+//   o_t = D_t (S q_t) + sum over j in P(t) of G(t, j) (k_j . q_t) u_j
+// that is: the 16 x 128 by 128 products S k_t and S q_t, all rows at once from registers; the rows' inner products; and a
+// triangular system of 16 unknowns per state row, one thread each. Chains and trees are the same formulas. The fold is the same
+// system over the pending rows, then one update of rank `pending`: S = D S + sum_t G(last, t) u_t k_t^T. One layer of the 27B
+// shape takes 13.6 us instead of 23.4, eight lanes 73 instead of 106 (the kernel alone, in a graph); the folded state's error
+// against 64 bits stays at 6e-8, and that of the rows' outputs at their bf16. What bounds it now is the prologue's latency
+// (dependent loads, the gate projection), four cluster barriers, and, with many lanes, instruction issue (half of the slots) and the
+// shared-memory port.
+//   CTA      256 threads; warp w owns rows 16 (w & 1).. of the CTA's 32 and key columns 32 (w / 2).. , in fp32 registers laid out as
+//            the tensor cores' A operand
 //   rollback the state after the block is never stored: the caller passes how many tape rows were accepted
 //            (pending_rows, or a device word written by sb_accept) to the next step, which folds them
 #include <algorithm>
-#include <atomic>
 #include <cooperative_groups.h>
 
 #include "sb_internal.h"
@@ -35,12 +49,10 @@ constexpr int kD = 128, kTaps = 4;
 
 struct GdnParams {
   SbGdnArgs a;
-  uint16_t *scratch;    // bf16 [value_heads][16][128] recurrent outputs before the gate
-  uint32_t *counters;   // [value_heads]
 };
 
 // Lane blockIdx.z's view of a launch over several lanes: its 16 row slots of the row-indexed buffers, its cell, tapes and
-// pending words, its share of the scratch and the counters.
+// pending words.
 __device__ __forceinline__ GdnParams gdn_lane_view(GdnParams p) {
   const uint32_t z = blockIdx.z;
   if (z == 0 && gridDim.z == 1) return p;
@@ -64,8 +76,6 @@ __device__ __forceinline__ GdnParams gdn_lane_view(GdnParams p) {
   tape(a.pending), tape(a.step);
   if (a.pending_rows_dev) a.pending_rows_dev += z;
   if (a.pending_path_dev) a.pending_path_dev += z;
-  p.scratch += size_t(z) * a.value_heads * 16 * 128;
-  p.counters += size_t(z) * a.value_heads;
   return p;
 }
 
@@ -81,403 +91,571 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// The kGdnSplit CTAs of a value head form a cluster: the fused gate projection is divided among them by rows and
-// meets in every CTA's shared memory.
-// kTree: the rows may form a tree and the pending path may be any row mask (tap tables, transformed queries); without
-// it the rows are a chain and the pending rows the tape's first, which is the verify step's usual case and keeps the
-// indirections out of its kernel.
-// kResident: CTAs per SM the registers are held to. A launch of one lane (192 CTAs on the 27B shape) runs fastest with the 96
-// registers that two per SM allow; a launch of several lanes has CTAs to spare, and four per SM at 64 registers hide more
-// of the chain's latency (measured on 8 lanes: the 27B step 25.95 ms at two per SM, 24.69 at three, 24.51 at four).
+// Sixteen values a lane, summed over the warp: lane l ends with value l >> 1 (both lanes of a pair hold it).
+__device__ __forceinline__ float sum_scatter16(float (&v)[16], uint32_t lane) {
+#pragma unroll
+  for (int half = 8; half; half >>= 1) {
+    const bool upper = (lane & (2 * half)) != 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i >= half) break;
+      const float give = upper ? v[i] : v[i + half], keep = upper ? v[i + half] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * half);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+template <int BYTES> __device__ __forceinline__ void copy_async(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+// Two neighbouring bf16 of a tape whose base need not lie on more than its element's two bytes.
+__device__ __forceinline__ uint32_t load_pair(const uint16_t *p) {
+  return (reinterpret_cast<uintptr_t>(p) & 3) == 0 ? *reinterpret_cast<const uint32_t *>(p) : uint32_t(p[0]) | (uint32_t(p[1]) << 16);
+}
+__device__ __forceinline__ void store_pair(uint16_t *p, uint32_t v) {
+  if ((reinterpret_cast<uintptr_t>(p) & 3) == 0) *reinterpret_cast<uint32_t *>(p) = v;
+  else p[0] = uint16_t(v), p[1] = uint16_t(v >> 16);
+}
+
+// Two floats as three bf16 terms each (hi + mid + lo carry the 24 bits of an fp32 significand), packed.
+__device__ __forceinline__ void split3(float a, float b, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  const float ar = a - __low2float(h), br = b - __high2float(h);
+  const __nv_bfloat162 m = __floats2bfloat162_rn(ar, br), l = __floats2bfloat162_rn(ar - __low2float(m), br - __high2float(m));
+  hi = *reinterpret_cast<const uint32_t *>(&h), mid = *reinterpret_cast<const uint32_t *>(&m), lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+
+constexpr int kKeyPitch = kD + 8, kPendingPitch = kD + 4, kProductPitch = 36, kGramPitch = 20;
+constexpr int kLocal = 2 * kD + kGdnVd;  // 288 channels of a CTA: q and k of the key head, 32 value dimensions
+struct GdnShared {
+  uint16_t x[2][kGdnRows][kKeyPitch];         // bf16 k rows, q rows
+  float pk[kGdnRows][kPendingPitch];
+  float v[kGdnRows][kGdnVd], pv[kGdnRows][kGdnVd];
+  union {
+    uint16_t in[kGdnRows + 3][kLocal];                 // convolution inputs, until the tape is written
+    float part[4][2 * kGdnRows][kProductPitch];        // then: the four column quarters' shares of S pk_t (pending rows), later of S k_t and S q_t
+  };
+  float u[kGdnRows][kGdnVd];                  // D_t (S k_t), then the solution: pending rows (scaled for the update), then the block's
+  float o[kGdnRows][kGdnVd];                  // D_t (S q_t), this CTA's value dimensions
+  float kk[kGdnRows][kGramPitch], kq[kGdnRows][kGramPitch], pkk[kGdnRows][kGramPitch];  // inner products [t][j] and coefficients (see there)
+  float out[kGdnRows / kGdnSplit][kD];        // outputs of the rows this CTA normalises
+  uint2 w[kLocal];
+  float gate[kDotGroups][kGdnRows][2];        // group partial sums of the head's b and a per row (fused gate projection)
+  alignas(16) float beta[kGdnRows], decay[kGdnRows], pbeta[kGdnRows], pdecay[kGdnRows];
+  alignas(16) float after[kGdnRows];          // products of the pending decays after a row
+  float pending_decay;                        // and of all of them
+  uint32_t path[kGdnRows];                    // the row's path from the anchor, itself included
+  uint8_t tap[kGdnRows][kTaps];               // where in `in` a row's four convolution taps lie (its path's last tokens)
+};
+static_assert(sizeof(GdnShared) <= 56 * 1024, "four CTAs a SM");
+static_assert(kGdnThreads / 32 == kDotGroups && kGdnThreads == kGdnRows * kGdnRows, "a warp a group of the dot product, a thread a coefficient");
+static_assert(kGdnRows == 4 * kGdnSplit, "four rows per CTA of the head");
+
+// kTree: the rows may form a tree and the pending path may be any row mask; without it the rows are a chain and the pending
+// rows the tape's first, which keeps the tap and path tables out of the usual case.
+// kResident: CTAs per SM the registers are held to: two for a launch of one lane (192 CTAs on the 27B shape), four for several.
+// Both run the same arithmetic: a lane's bits do not depend on the launch it is in.
 template <bool kTree, int kResident = 2>
 __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads, kResident) gdn_kernel(const GdnParams p_in) {
   const GdnParams p = gdn_lane_view(p_in);  // (one lane: p_in itself)
   const SbGdnArgs &a = p.a;
-  __shared__ float q_s[kGdnRows][kD], k_s[kGdnRows][kD], pk_s[kGdnRows][kD];
-  __shared__ float v_s[kGdnRows][kGdnVd], pv_s[kGdnRows][kGdnVd], o_s[kGdnRows][kGdnVd];
-  __shared__ float beta_s[kGdnRows], decay_s[kGdnRows], pbeta_s[kGdnRows], pdecay_s[kGdnRows];
-  __shared__ float gate_s[kDotGroups][kGdnRows][2];  // group partial sums of the head's b and a per row (fused gate projection)
-  __shared__ __align__(16) uint16_t in_s[kGdnRows + 3][2 * kD + kGdnVd];
-  __shared__ uint2 w_s[2 * kD + kGdnVd];
-  __shared__ uint32_t s_last;
-  __shared__ uint8_t tap_s[kGdnRows][kTaps];   // where in in_s a row's four convolution taps lie (its path's last tokens)
-  __shared__ uint32_t path_s[kGdnRows];         // the row's path from the anchor, itself included
-  __shared__ float coef_s[kGdnRows][kGdnRows];  // tree rows: the coefficient of each row of the path
+  extern __shared__ __align__(16) uint8_t gdn_smem[];
+  GdnShared &sh = *reinterpret_cast<GdnShared *>(gdn_smem);
+  namespace cg = cooperative_groups;
+  cg::cluster_group head_ctas = cg::this_cluster();
+  auto cluster_arrive = [] { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); };
+  auto cluster_wait = [] { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); };
   pdl_launch_dependents();
-  const bool fused_gates = a.gate_weight && a.rows > 0;
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // "this CTA runs", waited for before the first store into a peer CTA
-  bool peers_run = false;
-  auto wait_peers_run = [&] {
-    if (!peers_run) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    peers_run = true;
-  };
+  cluster_arrive();  // "this CTA runs", waited for before the first store into a peer CTA
   const uint32_t vs = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t KH = a.key_heads, VH = a.value_heads, KW = KH * kD, VW = VH * kD, C = 2 * KW + VW;
   const uint32_t per_key = VH / KH, kh = h / per_key, vd0 = vs * kGdnVd;
   const uint32_t rows = a.rows;
+  const bool fused_gates = a.gate_weight && rows > 0;
   const uint16_t *qkvz = static_cast<const uint16_t *>(a.qkvz);
   const uint16_t *conv_w = static_cast<const uint16_t *>(a.conv_w);
   const uint16_t *cs_in = static_cast<const uint16_t *>(a.conv_state_in);
   const uint16_t *pin = static_cast<const uint16_t *>(a.pending.inputs);
   const bool qk_writer = h % per_key == 0 && vs == 0;
 
-  // The state of this warp's 4 value dimensions, requested first so the latency hides behind the prologue and, where
+  // This warp's share of the state, requested first so the latency hides behind the prologue and, where
   // the caller allows it (below), before the wait for the kernel ahead: in the model's step the cell was written a
   // whole step ago, and this CTA may be resident while the projection before it drains.
-  // lane l holds row 4 warp + l / 8, key columns 32 c + 4 (l % 8) .. + 3 for c = 0..3 (the 8 lanes of a row read 128
-  // contiguous bytes at a time, from global and from shared memory), so a dot product over the 128 key columns
-  // is 16 multiply-adds in the lane and three butterfly rounds over its 8-lane group.
+  // The share is two 16 x 16 blocks as the tensor cores' A operand has them: rows 16 (warp & 1) + g and + 8 (g = lane / 4), key columns
+  // 32 (warp / 2) + 16 b + 2 t, + 1, + 8, + 9 (t = lane % 4) of blocks b = 0, 1; S[8 b + 4 (second row) + 2 (second pair) + i].
   float S[16];
-  const uint32_t srow = 4 * warp + (lane >> 3), scol = 4 * (lane & 7);
+  const uint32_t g4 = lane >> 2, t4 = lane & 3, quarter = warp >> 1, srow = 16 * (warp & 1) + g4, scol = 32 * quarter + 2 * t4;
   const size_t sbase = (size_t(h) * kD + vd0 + srow) * kD + scol;
   auto load_state = [&] {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float4 s4 = *reinterpret_cast<const float4 *>(a.state_in + sbase + 32 * c);
-      S[4 * c] = s4.x, S[4 * c + 1] = s4.y, S[4 * c + 2] = s4.z, S[4 * c + 3] = s4.w;
-    }
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int second = 0; second < 2; ++second)
+#pragma unroll
+        for (int pair = 0; pair < 2; ++pair) {
+          const float2 s2 = *reinterpret_cast<const float2 *>(a.state_in + sbase + size_t(8 * second) * kD + 16 * b + 8 * pair);
+          S[8 * b + 4 * second + 2 * pair] = s2.x, S[8 * b + 4 * second + 2 * pair + 1] = s2.y;
+        }
   };
   // Only a caller that vouches for the cell (SB_GDN_STATE_SETTLED: nothing still running on the stream writes
   // state_in) gets the early load; otherwise the launch ahead may be the one that produced the cell (a fold
   // followed at once by a step on the swapped cells), and the load waits for it like every other read.
+  const float a_scale = a.a_scale[h], dt_bias = bf16_bits_to_float(static_cast<const uint16_t *>(a.dt_bias)[h]);  // (weights)
   const bool settled = (a.flags & SB_GDN_STATE_SETTLED) != 0;
   if (settled) load_state();
   pdl_wait();
   if (!settled) load_state();
-  // The previous step's accepted path in its tape: a row mask, or the tape's first rows.
-  uint32_t pending_path = a.pending_path_dev ? *a.pending_path_dev : a.pending_path;
-  if (!a.pending_path_dev && !a.pending_path) {
-    const uint32_t n = a.pending_rows_dev ? min(*a.pending_rows_dev, uint32_t(kGdnRows)) : a.pending_rows;
-    pending_path = (1u << n) - 1u;
+  // Conv inputs of this CTA's channels (q and k of the key head, 32 value dimensions), in[3 + row][local channel], and their taps'
+  // weights: asynchronous copies, on their way while the gate projection runs.
+  const uint32_t chan0[3] = {kh * kD, KW + kh * kD, 2 * KW + h * kD + vd0};
+  auto global_channel = [&](uint32_t lc) { return lc < kD ? chan0[0] + lc : lc < 2 * kD ? chan0[1] + lc - kD : chan0[2] + lc - 2 * kD; };
+  uint32_t pending_path = a.pending_path_dev ? *a.pending_path_dev : a.pending_path;  // (first used below the gate projection)
+  uint32_t pending_n = a.pending_rows_dev ? *a.pending_rows_dev : a.pending_rows;
+  for (uint32_t i = tid; i < rows * (kLocal / 8); i += kGdnThreads) {
+    const uint32_t r = i / (kLocal / 8), lc = (i % (kLocal / 8)) * 8;
+    copy_async<16>(&sh.in[3 + r][lc], qkvz + size_t(r) * a.qkvz_stride + global_channel(lc));
   }
-  pending_path &= (1u << kGdnRows) - 1u;
-  const uint32_t pending = uint32_t(__popc(pending_path));
-  auto pending_row = [&](uint32_t n) { return kTree ? path_row(pending_path, n) : n; };
-  if (kTree && tid < rows) {
-    const uint32_t path = (a.tree ? static_cast<const uint2 *>(a.tree)[tid].x & ((2u << tid) - 1u) : (2u << tid) - 1u) | (1u << tid);
-    const int depth = __popc(path) - 1;
-    for (int tap = 0; tap < kTaps; ++tap) {
-      const int at = depth - 3 + tap;  // the tap's token, counted from the anchor; before it: the carried history
-      tap_s[tid][tap] = uint8_t(at < 0 ? 3 + at : 3 + int(path_row(path, uint32_t(at))));
+  for (uint32_t lc = tid; lc < kLocal; lc += kGdnThreads) copy_async<8>(&sh.w[lc], conv_w + size_t(global_channel(lc)) * kTaps);
+  if (tid < kGdnRows) {
+    uint32_t path = (2u << tid) - 1u;
+    if (kTree && tid < rows) {
+      path = (a.tree ? static_cast<const uint2 *>(a.tree)[tid].x & path : path) | (1u << tid);
+      const int depth = __popc(path) - 1;
+      for (int tap = 0; tap < kTaps; ++tap) {
+        const int at = depth - 3 + tap;  // the tap's token, counted from the anchor; before it: the carried history
+        sh.tap[tid][tap] = uint8_t(at < 0 ? 3 + at : 3 + int(path_row(path, uint32_t(at))));
+      }
     }
-    path_s[tid] = path;
+    sh.path[tid] = path;
   }
   // Fused gate projection: this CTA takes rows 4 vs .. 4 vs + 3; warp w computes group w's partial sums of those rows x
   // {b, a} over the layer's normalised input and stores them into all four CTAs of the head; the rows' threads add the
   // 8 groups in order below (the order of sb_linear_f32, so the bits agree with the unfused way).
+  float gates[4][2];
   if (fused_gates) {
-    static_assert(kGdnThreads / 32 == kDotGroups, "one warp per group of the dot product");
-    static_assert(kGdnRows == 4 * kGdnSplit, "four rows of the gate projection per CTA of the head");
     const float *const wrow[2] = {a.gate_weight + size_t(h) * a.gate_k, a.gate_weight + size_t(VH + h) * a.gate_k};
     const uint16_t *gx = static_cast<const uint16_t *>(a.gate_input);
     const uint16_t *xrow[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) xrow[r] = gx + size_t(min(4 * vs + uint32_t(r), rows - 1)) * a.gate_input_stride;
-    float d[4][2];
-    warp_dot_group_f32_bf16<2, 4>(wrow, xrow, a.gate_k, lane, warp, d);
-    wait_peers_run();
-    if (lane < kGdnSplit) {
-      cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-      float *remote = cluster.map_shared_rank(&gate_s[0][0][0], lane);
+    lane_dot_group_f32_bf16<2, 4>(wrow, xrow, a.gate_k, lane, warp, gates);
+  }
+  // The previous step's accepted path in its tape: a row mask, or the tape's first rows.
+  if (!a.pending_path_dev && !a.pending_path) pending_path = (1u << min(pending_n, uint32_t(kGdnRows))) - 1u;
+  pending_path &= (1u << kGdnRows) - 1u;
+  const uint32_t pending = uint32_t(__popc(pending_path));
+  auto pending_row = [&](uint32_t n) { return kTree ? path_row(pending_path, n) : n; };
+  // History rows -3..-1: row i (0..2, oldest first) is row pending - 3 + i of (carried rows ++ pending rows).
+  if (tid < 3 * (kLocal / 8)) {
+    const uint32_t r = tid / (kLocal / 8), lc = (tid % (kLocal / 8)) * 8, ch = global_channel(lc);
+    const int hsrc = int(pending) - 3 + int(r);
+    copy_async<16>(&sh.in[r][lc], hsrc >= 0 ? pin + size_t(pending_row(uint32_t(hsrc))) * C + ch : cs_in + size_t(3 + hsrc) * C + ch);
+  }
+  // pending rows' keys, values and gates from their tape, requested before the gate projection's lanes are added up and stored
+  // after; rows past them are zeros (the products below take whole eights)
+  constexpr int kPkLoads = kGdnRows * kD / 2 / kGdnThreads, kPvLoads = kGdnRows * kGdnVd / kGdnThreads;
+  uint32_t pk2[kPkLoads];
+  uint16_t pv1[kPvLoads], pbeta1 = 0;
+  float pdecay1 = 0.0f;
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        remote[(warp * kGdnRows + 4 * vs + r) * 2] = d[r][0];
-        remote[(warp * kGdnRows + 4 * vs + r) * 2 + 1] = d[r][1];
-      }
-    }
+  for (int i = 0; i < kPkLoads; ++i) {
+    const uint32_t n = tid / (kD / 2) + i * (kGdnThreads / (kD / 2)), d = 2 * (tid % (kD / 2));
+    pk2[i] = n < pending ? load_pair(static_cast<const uint16_t *>(a.pending.k) + size_t(pending_row(n)) * KW + kh * kD + d) : 0u;
   }
-  // Conv inputs of this CTA's channels (q and k of the key head, 32 value dimensions) for history rows
-  // -3..-1 and the block's rows, staged with 16-byte loads: in_s[3 + row][local channel]. History row i
-  // (0..2, oldest first) is row pending - 3 + i of (carried rows ++ pending rows).
-  constexpr int kLocal = 2 * kD + kGdnVd;  // 288 local channels
-  const uint32_t chan0[3] = {kh * kD, KW + kh * kD, 2 * KW + h * kD + vd0};
-  auto global_channel = [&](uint32_t lc) { return lc < kD ? chan0[0] + lc : lc < 2 * kD ? chan0[1] + lc - kD : chan0[2] + lc - 2 * kD; };
-  for (uint32_t i = tid; i < (3 + rows) * (kLocal / 8); i += kGdnThreads) {
-    const uint32_t r = i / (kLocal / 8), lc = (i % (kLocal / 8)) * 8, ch = global_channel(lc);
-    const uint16_t *src;
-    if (r >= 3) {
-      src = qkvz + size_t(r - 3) * a.qkvz_stride + ch;
-    } else {
-      const int hsrc = int(pending) - 3 + int(r);
-      src = hsrc >= 0 ? pin + size_t(pending_row(uint32_t(hsrc))) * C + ch : cs_in + size_t(3 + hsrc) * C + ch;
-    }
-    *reinterpret_cast<uint4 *>(&in_s[r][lc]) = *reinterpret_cast<const uint4 *>(src);
-  }
-  for (uint32_t lc = tid; lc < kLocal; lc += kGdnThreads)
-    w_s[lc] = *reinterpret_cast<const uint2 *>(conv_w + size_t(global_channel(lc)) * kTaps);
-  if (fused_gates) cooperative_groups::this_cluster().sync();  // the gates of all rows are here (and the CTA's staging is complete)
-  else __syncthreads();
-  auto conv = [&](uint32_t row, uint32_t lc) -> float {
-    const uint2 wv = w_s[lc];
-    const float w[4] = {bf16_bits_to_float(wv.x & 0xffffu), bf16_bits_to_float(wv.x >> 16), bf16_bits_to_float(wv.y & 0xffffu),
-                        bf16_bits_to_float(wv.y >> 16)};
-    float value = 0.0f;
 #pragma unroll
-    for (int tap = 0; tap < kTaps; ++tap) value = __fadd_rn(value, __fmul_rn(bf16_bits_to_float(in_s[kTree ? uint32_t(tap_s[row][tap]) : row + tap][lc]), w[tap]));
-    value = round_bf16(value);
-    return round_bf16(silu_f(value));
-  };
-
-  // (2) conv outputs: this CTA's 32 value dimensions, and q, k of the key head (128 each) for rows 4 vs .. 4 vs + 3 only:
-  // the head's four CTAs divide the rows, normalise their own and store the result into all four (below).
-  const uint32_t qk_row0 = min(4 * vs, rows), qk_rows = min(4 * vs + 4, rows) - qk_row0;
-#pragma unroll 2
-  for (uint32_t i = tid; i < qk_rows * kD; i += kGdnThreads) {
-    const uint32_t r = qk_row0 + i / kD, d = i % kD;
-    q_s[r][d] = conv(r, d);
-    k_s[r][d] = conv(r, kD + d);
+  for (int i = 0; i < kPvLoads; ++i) {
+    const uint32_t n = warp + i * (kGdnThreads / kGdnVd);
+    pv1[i] = n < pending ? static_cast<const uint16_t *>(a.pending.v)[size_t(pending_row(n)) * VW + h * kD + vd0 + lane] : uint16_t(0);
   }
-#pragma unroll 2
-  for (uint32_t i = tid; i < rows * kGdnVd; i += kGdnThreads) {
-    const uint32_t r = i / kGdnVd, d = i % kGdnVd;
-    v_s[r][d] = conv(r, 2 * kD + d);
-  }
-  // pending rows' keys, values and gates from their tape
-  for (uint32_t i = tid; i < pending * kD; i += kGdnThreads)
-    pk_s[i / kD][i % kD] =
-        bf16_bits_to_float(static_cast<const uint16_t *>(a.pending.k)[size_t(pending_row(i / kD)) * KW + kh * kD + i % kD]);
-  for (uint32_t i = tid; i < pending * kGdnVd; i += kGdnThreads)
-    pv_s[i / kGdnVd][i % kGdnVd] = bf16_bits_to_float(
-        static_cast<const uint16_t *>(a.pending.v)[size_t(pending_row(i / kGdnVd)) * VW + h * kD + vd0 + i % kGdnVd]);
   if (tid < pending) {
     const uint32_t trow = pending_row(tid);
-    pbeta_s[tid] = bf16_bits_to_float(static_cast<const uint16_t *>(a.pending.beta)[size_t(trow) * VH + h]);
-    pdecay_s[tid] = a.pending.decay[size_t(trow) * VH + h];
+    pbeta1 = static_cast<const uint16_t *>(a.pending.beta)[size_t(trow) * VH + h], pdecay1 = a.pending.decay[size_t(trow) * VH + h];
   }
-  if (tid < rows) {
-    float bb, aa;
-    if (a.gate_weight) {
-      bb = gate_s[0][tid][0], aa = gate_s[0][tid][1];
+  // The gates' eight sums over the lanes, halved at every exchange: lane l ends with sum l / 4 (row l / 8, b or a). The same
+  // additions as a butterfly of each, so the same bits.
+  float gate_sum = 0.0f;
+  if (fused_gates) {
+    float v[8];
 #pragma unroll
-      for (int g = 1; g < kDotGroups; ++g) bb += gate_s[g][tid][0], aa += gate_s[g][tid][1];
-      bb = round_bf16(bb), aa = round_bf16(aa);
-    } else {
-      bb = bf16_bits_to_float(static_cast<const uint16_t *>(a.b)[size_t(tid) * a.ab_stride + h]);
-      aa = bf16_bits_to_float(static_cast<const uint16_t *>(a.a)[size_t(tid) * a.ab_stride + h]);
+    for (int i = 0; i < 8; ++i) v[i] = gates[i >> 1][i & 1];
+#pragma unroll
+    for (int half = 4; half; half >>= 1) {
+      const bool upper = (lane & (4 * half)) != 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i >= half) break;
+        const float give = upper ? v[i] : v[i + half], keep = upper ? v[i + half] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * half);
+      }
     }
-    const float be = round_bf16(sigmoid_f(bb));
-    const float x = round_bf16(__fadd_rn(aa, bf16_bits_to_float(static_cast<const uint16_t *>(a.dt_bias)[h])));
-    const float sp = round_bf16(fmaxf(x, 0.0f) + log2f(1.0f + exp2f(-1.44269504089f * fabsf(x))) * 0.69314718056f);
-    const float de = expf(a.a_scale[h] * sp);
-    beta_s[tid] = be;
-    decay_s[tid] = de;
-    if (vs == 0) {
-      static_cast<uint16_t *>(a.step.beta)[size_t(tid) * VH + h] = float_to_bf16_bits(be);
-      a.step.decay[size_t(tid) * VH + h] = de;
-    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    gate_sum = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
   }
-  __syncthreads();
-  // q/k RMS norm over the head's 128 dimensions: a warp per (row, q or k); 4 dims per lane in order,
-  // then the butterfly.
-  wait_peers_run();
-  cooperative_groups::cluster_group head_ctas = cooperative_groups::this_cluster();
-  for (uint32_t task = warp; task < 2 * qk_rows; task += kGdnThreads / 32) {
-    const uint32_t r = qk_row0 + (task >> 1);
-    float *vec = (task & 1) ? k_s[r] : q_s[r];
-    float ss = 0.0f;
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      const float x = vec[32 * g + lane];
-      ss += warp_sum(x * x);
+  for (int i = 0; i < kPkLoads; ++i) {
+    const uint32_t n = tid / (kD / 2) + i * (kGdnThreads / (kD / 2));
+    *reinterpret_cast<float2 *>(&sh.pk[n][2 * (tid % (kD / 2))]) = make_float2(bf16_bits_to_float(pk2[i] & 0xffffu), bf16_bits_to_float(pk2[i] >> 16));
+  }
+#pragma unroll
+  for (int i = 0; i < kPvLoads; ++i) sh.pv[warp + i * (kGdnThreads / kGdnVd)][lane] = bf16_bits_to_float(pv1[i]);
+  if (tid < kGdnRows) sh.pbeta[tid] = bf16_bits_to_float(pbeta1), sh.pdecay[tid] = pdecay1;
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  // The sixteen inner products of a row with rows of keys, into row t of every CTA's matrix: a warp, four dimensions a lane.
+  auto inner_products = [&](auto key, const float4 x4, float (*gram)[kGramPitch], uint32_t t) {
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float4 k4 = key(j);
+      v[j] = fmaf(k4.w, x4.w, fmaf(k4.z, x4.z, fmaf(k4.y, x4.y, k4.x * x4.x)));
     }
+    const float dot = sum_scatter16(v, lane);
+    const uint32_t j = lane >> 1;
+    // (the pair's two lanes store to two CTAs each)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) head_ctas.map_shared_rank(&gram[t][j], int(2 * (lane & 1) + half))[0] = dot;
+  };
+  auto pending_key = [&](int j) { return *reinterpret_cast<const float4 *>(&sh.pk[j][4 * lane]); };
+  auto block_row = [&](int which, int j) {
+    const uint2 two = *reinterpret_cast<const uint2 *>(&sh.x[which][j][4 * lane]);
+    return make_float4(bf16_bits_to_float(two.x & 0xffffu), bf16_bits_to_float(two.x >> 16), bf16_bits_to_float(two.y & 0xffffu), bf16_bits_to_float(two.y >> 16));
+  };
+  __syncthreads();  // the CTA's staging is complete
+  cluster_wait();   // every CTA of the head runs
+  if (fused_gates) head_ctas.map_shared_rank(&sh.gate[warp][4 * vs + (lane >> 3)][(lane >> 2) & 1], int(lane & 3))[0] = gate_sum;
+  if (warp >= 4 && 4 * (warp - 4) + vs < pending) inner_products(pending_key, pending_key(4 * (warp - 4) + vs), sh.pkk, 4 * (warp - 4) + vs);
+  cluster_arrive();  // (1) the gates' sums and the pending rows' inner products
+  // NC neighbouring channels' convolution and SiLU for a row.
+  auto conv = [&](uint32_t row, uint32_t lc, auto &out) {
+    constexpr int NC = sizeof(out) / sizeof(float);
+    uint2 wv[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) wv[c] = sh.w[lc + c];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) out[c] = 0.0f;
+#pragma unroll
+    for (int tap = 0; tap < kTaps; ++tap) {
+      const uint16_t *x = &sh.in[kTree ? uint32_t(sh.tap[row][tap]) : row + tap][lc];
+      uint32_t two[NC / 2];
+      if (NC == 4) {
+        const uint2 t = *reinterpret_cast<const uint2 *>(x);
+        two[0] = t.x, two[NC / 2 - 1] = t.y;
+      } else {
+        two[0] = *reinterpret_cast<const uint32_t *>(x);
+      }
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const uint32_t pair = tap < 2 ? wv[c].x : wv[c].y;
+        const float w = bf16_bits_to_float((tap & 1) ? pair >> 16 : pair & 0xffffu);
+        out[c] = __fadd_rn(out[c], __fmul_rn(bf16_bits_to_float((c & 1) ? two[c / 2] >> 16 : two[c / 2] & 0xffffu), w));
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) out[c] = round_bf16(silu_f(round_bf16(out[c])));
+  };
+  // (2) conv outputs: this CTA's 32 value dimensions, and q, k of the key head (128 each) for rows 4 vs .. 4 vs + 3 only:
+  // the head's four CTAs divide the rows, normalise their own and store the result into all four. A warp takes q or k of a row,
+  // four dimensions a lane, so its convolution, norm and stores need nobody else.
+  const uint32_t qk_row = 4 * vs + (warp >> 1);
+  if (qk_row < rows) {
+    float x[4];
+    conv(qk_row, ((warp & 1) ? kD : 0) + 4 * lane, x);
+    const float ss = warp_sum((x[0] * x[0] + x[1] * x[1]) + (x[2] * x[2] + x[3] * x[3]));
     const float inv = rsqrtf(ss / float(kD) + 1e-6f);
-    const float post = (task & 1) ? 0.08838834765f : 0.0078125f;
-    float out[4];
+    const float post = (warp & 1) ? 0.08838834765f : 0.0078125f;
+    uint32_t bits[2];
 #pragma unroll
-    for (int g = 0; g < 4; ++g) out[g] = round_bf16(round_bf16(vec[32 * g + lane] * inv) * post);
+    for (int i = 0; i < 2; ++i)
+      bits[i] = uint32_t(float_to_bf16_bits(round_bf16(x[2 * i] * inv) * post)) | (uint32_t(float_to_bf16_bits(round_bf16(x[2 * i + 1] * inv) * post)) << 16);
+    uint16_t *vec = &sh.x[(warp & 1) ? 0 : 1][qk_row][4 * lane];
 #pragma unroll
-    for (int peer = 0; peer < kGdnSplit; ++peer) {
-      float *remote = head_ctas.map_shared_rank(vec, peer);
-#pragma unroll
-      for (int g = 0; g < 4; ++g) remote[32 * g + lane] = out[g];
-    }
+    for (int peer = 0; peer < kGdnSplit; ++peer) *reinterpret_cast<uint2 *>(head_ctas.map_shared_rank(vec, peer)) = make_uint2(bits[0], bits[1]);
   }
-  head_ctas.sync();  // every row's q and k are in every CTA of the head
-  // (6) tape and carried conv rows, from the staged inputs.
+  // (rows past the block are zeros: the products take all sixteen)
+  for (uint32_t i = tid; i < (kGdnRows - rows) * (kD / 2); i += kGdnThreads)
+    *reinterpret_cast<uint32_t *>(&sh.x[0][rows + i / (kD / 2)][2 * (i % (kD / 2))]) = *reinterpret_cast<uint32_t *>(&sh.x[1][rows + i / (kD / 2)][2 * (i % (kD / 2))]) = 0u;
+  // Two values of a row a thread, here and below: row ct, value dimensions 2 cj, + 1.
+  const uint32_t ct = tid / kGdnRows, cj = tid % kGdnRows, cv = 2 * cj;
+  if (ct >= rows) {
+    *reinterpret_cast<float2 *>(&sh.v[ct][cv]) = make_float2(0.0f, 0.0f);  // (and no gate, below: no update)
+  } else {
+    float v[2];
+    conv(ct, 2 * kD + cv, v);
+    *reinterpret_cast<float2 *>(&sh.v[ct][cv]) = make_float2(v[0], v[1]);
+    store_pair(static_cast<uint16_t *>(a.step.v) + size_t(ct) * VW + h * kD + vd0 + cv, uint32_t(float_to_bf16_bits(v[0])) | (uint32_t(float_to_bf16_bits(v[1])) << 16));
+  }
+  // (6) this step's tape of inputs and the carried conv rows, from the staged inputs (the value channels, and the key head's in
+  // one CTA), eight channels at a time
   {
     uint16_t *tin = static_cast<uint16_t *>(a.step.inputs), *cs_out = static_cast<uint16_t *>(a.conv_state_out);
-    for (uint32_t i = tid; i < (3 + rows) * kLocal; i += kGdnThreads) {
-      const uint32_t r = i / kLocal, lc = i % kLocal;
-      if (lc < 2 * kD && !qk_writer) continue;
-      const uint32_t ch = global_channel(lc);
-      if (r < 3) cs_out[size_t(r) * C + ch] = in_s[r][lc];
-      else tin[size_t(r - 3) * C + ch] = in_s[r][lc];
+    const uint32_t lc0 = qk_writer ? 0 : 2 * kD, units = (kLocal - lc0) / 8;
+    for (uint32_t i = tid; i < (3 + rows) * units; i += kGdnThreads) {
+      const uint32_t r = i / units, lc = lc0 + 8 * (i % units), ch = global_channel(lc);
+      uint16_t *dst = r < 3 ? cs_out + size_t(r) * C + ch : tin + size_t(r - 3) * C + ch;
+      if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(&sh.in[r][lc]);
+      } else {  // (a tape or cell that lies on its element's two bytes only)
+#pragma unroll 1
+        for (int e = 0; e < 8; ++e) dst[e] = sh.in[r][lc + e];
+      }
     }
-    for (uint32_t i = tid; i < rows * kGdnVd; i += kGdnThreads)
-      static_cast<uint16_t *>(a.step.v)[size_t(i / kGdnVd) * VW + h * kD + vd0 + i % kGdnVd] = float_to_bf16_bits(v_s[i / kGdnVd][i % kGdnVd]);
-    if (qk_writer)
-      for (uint32_t i = tid; i < rows * kD; i += kGdnThreads)
-        static_cast<uint16_t *>(a.step.k)[size_t(i / kD) * KW + kh * kD + i % kD] = float_to_bf16_bits(k_s[i / kD][i % kD]);
   }
-
-  // (3) + (4): one delta-rule step on the lane's 16 state values (runtime/metal/kernels/common/gdn_primitives.h:63-97):
-  // S *= decay; mem = S k; delta = (v - mem) beta; S += delta k^T; out = S q.
-  auto group_sum = [&](float v) {
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
-    return v;
+  cluster_wait();  // (1)
+  auto four = [&](const float (&m)[4][2 * kGdnRows][kProductPitch], uint32_t i) {  // the quarters in order
+    const float2 p0 = *reinterpret_cast<const float2 *>(&m[0][i][cv]), p1 = *reinterpret_cast<const float2 *>(&m[1][i][cv]);
+    const float2 p2 = *reinterpret_cast<const float2 *>(&m[2][i][cv]), p3 = *reinterpret_cast<const float2 *>(&m[3][i][cv]);
+    return make_float2(((p0.x + p1.x) + p2.x) + p3.x, ((p0.y + p1.y) + p2.y) + p3.y);
   };
-  auto advance = [&](const float *key, const float *val, float d, float b, const float *query, float *out) {
-    float kk[16];
+  // Product of the decays of the rows in a mask, in row order.
+  auto decays = [&](const float (&d)[kGdnRows], uint32_t mask) {
+    float g = 1.0f;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float4 k4 = *reinterpret_cast<const float4 *>(key + scol + 32 * c);
-      kk[4 * c] = k4.x, kk[4 * c + 1] = k4.y, kk[4 * c + 2] = k4.z, kk[4 * c + 3] = k4.w;
+    for (int i4 = 0; i4 < kGdnRows; i4 += 4) {
+      const float4 d4 = *reinterpret_cast<const float4 *>(&d[i4]);
+      g *= (mask >> i4 & 1u) ? d4.x : 1.0f, g *= (mask >> (i4 + 1) & 1u) ? d4.y : 1.0f;
+      g *= (mask >> (i4 + 2) & 1u) ? d4.z : 1.0f, g *= (mask >> (i4 + 3) & 1u) ? d4.w : 1.0f;
     }
-    float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    return g;
+  };
+  // The unknowns of state row `lane`, by one warp: u_t = beta_t (v_t - m_t), m_t = D_t (S k_t) (in sh.u) + sum over j < t of c[j][t] u_j,
+  // a finished unknown at a time so that a step waits for three operations only. What the state already holds of v_t is summed by
+  // itself: it is small beside v_t, so its roundings are too (with -beta c u_j added to the right-hand side one by one the folded
+  // state was 8e-8 off instead of 6e-8).
+  auto solve = [&](const float (*c)[kGramPitch], const float (&v)[kGdnRows][kGdnVd], const float (&beta)[kGdnRows], float (&u)[kGdnRows]) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      S[i] *= d;
-      part[i & 3] = fmaf(S[i], kk[i], part[i & 3]);
-    }
-    const float mem = group_sum((part[0] + part[1]) + (part[2] + part[3]));
-    const float delta = (val[srow] - mem) * b;
-    if (query) {
-      float qq[16];
+    for (int t = 0; t < kGdnRows; ++t) u[t] = sh.u[t][lane];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float4 q4 = *reinterpret_cast<const float4 *>(query + scol + 32 * c);
-        qq[4 * c] = q4.x, qq[4 * c + 1] = q4.y, qq[4 * c + 2] = q4.z, qq[4 * c + 3] = q4.w;
+    for (int j = 0; j < kGdnRows; ++j) {
+      u[j] = beta[j] * (v[j][lane] - u[j]);
+#pragma unroll
+      for (int t4x = (j + 1) / 4 * 4; t4x < kGdnRows; t4x += 4) {
+        const float4 c4 = *reinterpret_cast<const float4 *>(&c[j][t4x]);
+        if (t4x > j) u[t4x] = fmaf(c4.x, u[j], u[t4x]);
+        if (t4x + 1 > j) u[t4x + 1] = fmaf(c4.y, u[j], u[t4x + 1]);
+        if (t4x + 2 > j) u[t4x + 2] = fmaf(c4.z, u[j], u[t4x + 2]);
+        if (t4x + 3 > j) u[t4x + 3] = fmaf(c4.w, u[j], u[t4x + 3]);
       }
-      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        S[i] = fmaf(kk[i], delta, S[i]);
-        acc[i & 3] = fmaf(S[i], qq[i], acc[i & 3]);
-      }
-      const float res = group_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
-      if ((lane & 7) == 0) out[srow] = res;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) S[i] = fmaf(kk[i], delta, S[i]);
     }
   };
-  for (uint32_t t = 0; t < pending; ++t) advance(pk_s[t], pv_s[t], pdecay_s[t], pbeta_s[t], nullptr, nullptr);
+  if (pending) {  // (3)
+    __syncthreads();  // nobody reads the convolution inputs any more (they have been read since the CTA arrived)
+    // S pk_t: eight rows at a time, a thread its two state rows over its eight columns, summed over the four lanes that share
+    // the rows (products halved at every exchange).
+    for (uint32_t n0 = 0; n0 < pending; n0 += 8) {
+      float v[16];  // [row of the pair][pending row]
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
-    *reinterpret_cast<float4 *>(a.state_out + sbase + 32 * c) = make_float4(S[4 * c], S[4 * c + 1], S[4 * c + 2], S[4 * c + 3]);
-  bool chain = true;
-  if (kTree)
-    for (uint32_t r = 0; r < rows; ++r) chain = chain && path_s[r] == (2u << r) - 1u;
-  if (!kTree || chain) {
-    for (uint32_t t = 0; t < rows; ++t) advance(k_s[t], v_s[t], decay_s[t], beta_s[t], q_s[t], o_s[t]);
-  } else {
-    // Tree rows (runtime/metal/kernels/decode/gdn.metal:418-478): a row's output is the state after its own path,
-    // S_committed z + sum_j c_j v_j, with the query taken up the path: c_j = beta_j (k_j . z_j), z_j-1 = d_j (z_j - c_j k_j).
-    // A warp transforms rows warp and warp + 8 (four dimensions a lane); the transformed queries take the queries' place.
-    float z[2][4], cf[2] = {0.0f, 0.0f};
+      for (int n = 0; n < 8; ++n) {
+        float lo = 0.0f, hi = 0.0f;
 #pragma unroll
-    for (int pass = 0; pass < 2; ++pass) {
-      const uint32_t r = warp + 8 * pass;
-      if (r >= rows) continue;
-      const float4 q4 = *reinterpret_cast<const float4 *>(&q_s[r][4 * lane]);
-      z[pass][0] = q4.x, z[pass][1] = q4.y, z[pass][2] = q4.z, z[pass][3] = q4.w;
-      for (uint32_t up = path_s[r]; up;) {
-        const uint32_t row = 31u - uint32_t(__clz(int(up)));
-        up &= ~(1u << row);
-        const float4 k4 = *reinterpret_cast<const float4 *>(&k_s[row][4 * lane]);
-        const float c = beta_s[row] * warp_sum(k4.x * z[pass][0] + k4.y * z[pass][1] + k4.z * z[pass][2] + k4.w * z[pass][3]);
-        const float d = decay_s[row];
-        z[pass][0] = d * (z[pass][0] - c * k4.x), z[pass][1] = d * (z[pass][1] - c * k4.y);
-        z[pass][2] = d * (z[pass][2] - c * k4.z), z[pass][3] = d * (z[pass][3] - c * k4.w);
-        if (lane == row) cf[pass] = c;
+        for (int c = 0; c < 4; ++c) {  // block c / 2, pair c % 2
+          const float2 k2 = *reinterpret_cast<const float2 *>(&sh.pk[n0 + n][scol + 16 * (c >> 1) + 8 * (c & 1)]);
+          const int at = 8 * (c >> 1) + 2 * (c & 1);
+          lo = fmaf(S[at], k2.x, lo), lo = fmaf(S[at + 1], k2.y, lo);
+          hi = fmaf(S[at + 4], k2.x, hi), hi = fmaf(S[at + 5], k2.y, hi);
+        }
+        v[n] = lo, v[8 + n] = hi;
       }
-    }
-    __syncthreads();  // every warp has read the queries it needs
 #pragma unroll
-    for (int pass = 0; pass < 2; ++pass) {
-      const uint32_t r = warp + 8 * pass;
-      if (r >= rows) continue;
-      *reinterpret_cast<float4 *>(&q_s[r][4 * lane]) = make_float4(z[pass][0], z[pass][1], z[pass][2], z[pass][3]);
-      if (lane < kGdnRows) coef_s[r][lane] = cf[pass];
+      for (int half = 8; half >= 4; half >>= 1) {  // lanes 2 apart divide the pair's rows, lanes 1 apart the eight products
+        const bool upper = (lane & (half >> 2)) != 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (i >= half) break;
+          const float give = upper ? v[i] : v[i + half], keep = upper ? v[i + half] : v[i];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, give, half >> 2);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sh.part[quarter][n0 + 4 * (lane & 1) + i][srow + ((lane & 2) ? 8 : 0)] = v[i];
     }
     __syncthreads();
-    for (uint32_t t = 0; t < rows; ++t) {
-      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    // coefficients [j][t] (into the matrix the block's rows use later) and D_t (S k_t); rows past the pending ones are zeros
+    const bool there = ct < pending;
+    const uint32_t below = there ? (2u << ct) - 1u : 0u;
+    sh.kk[cj][ct] = there && cj < ct ? decays(sh.pdecay, below & ~((2u << cj) - 1u)) * sh.pkk[ct][cj] : 0.0f;
+    float2 right = make_float2(0.0f, 0.0f);
+    if (there) {
+      const float2 sx = four(sh.part, ct);
+      const float d = decays(sh.pdecay, below);
+      right = make_float2(d * sx.x, d * sx.y);
+    }
+    *reinterpret_cast<float2 *>(&sh.u[ct][cv]) = right;
+    if (cj == 0) sh.after[ct] = decays(sh.pdecay, ((1u << pending) - 1u) & ~((2u << ct) - 1u));
+    if (tid == 1) sh.pending_decay = decays(sh.pdecay, (1u << pending) - 1u);
+    __syncthreads();
+    if (warp == 0) {
+      float u[kGdnRows];
+      solve(sh.kk, sh.pv, sh.pbeta, u);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float4 q4 = *reinterpret_cast<const float4 *>(&q_s[t][scol + 32 * c]);
-        acc[0] = fmaf(S[4 * c], q4.x, acc[0]), acc[1] = fmaf(S[4 * c + 1], q4.y, acc[1]);
-        acc[2] = fmaf(S[4 * c + 2], q4.z, acc[2]), acc[3] = fmaf(S[4 * c + 3], q4.w, acc[3]);
+      for (int t4x = 0; t4x < kGdnRows; t4x += 4) {
+        const float4 g4x = *reinterpret_cast<const float4 *>(&sh.after[t4x]);
+        sh.u[t4x][lane] = g4x.x * u[t4x], sh.u[t4x + 1][lane] = g4x.y * u[t4x + 1];
+        sh.u[t4x + 2][lane] = g4x.z * u[t4x + 2], sh.u[t4x + 3][lane] = g4x.w * u[t4x + 3];
       }
-      float res = group_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
-      if ((lane & 7) == 0) {
-        for (uint32_t up = path_s[t]; up; up &= up - 1) {
-          const uint32_t j = uint32_t(__ffs(int(up))) - 1u;
-          res = fmaf(coef_s[t][j], v_s[j][srow], res);
+    }
+  }
+  if (warp == 1 && lane >= rows && lane < kGdnRows) sh.beta[lane] = 0.0f;
+  if (warp == 1 && lane < rows) {  // the rows' gates
+    float bb, aa;
+    if (a.gate_weight) {
+      bb = sh.gate[0][lane][0], aa = sh.gate[0][lane][1];
+#pragma unroll
+      for (int g = 1; g < kDotGroups; ++g) bb += sh.gate[g][lane][0], aa += sh.gate[g][lane][1];
+      bb = round_bf16(bb), aa = round_bf16(aa);
+    } else {
+      bb = bf16_bits_to_float(static_cast<const uint16_t *>(a.b)[size_t(lane) * a.ab_stride + h]);
+      aa = bf16_bits_to_float(static_cast<const uint16_t *>(a.a)[size_t(lane) * a.ab_stride + h]);
+    }
+    const float be = round_bf16(sigmoid_f(bb));
+    const float x = round_bf16(__fadd_rn(aa, dt_bias));
+    const float sp = round_bf16(fmaxf(x, 0.0f) + log2f(1.0f + exp2f(-1.44269504089f * fabsf(x))) * 0.69314718056f);
+    const float de = expf(a_scale * sp);
+    sh.beta[lane] = be;
+    sh.decay[lane] = de;
+    if (vs == 0) {
+      static_cast<uint16_t *>(a.step.beta)[size_t(lane) * VH + h] = float_to_bf16_bits(be);
+      a.step.decay[size_t(lane) * VH + h] = de;
+    }
+  }
+  cluster_arrive();
+  cluster_wait();  // (2) every row's q and k are in every CTA of the head; this CTA's pending solution and gates
+  if (pending) {
+    const float d = sh.pending_decay;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) S[i] *= d;
+    for (uint32_t t0 = 0; t0 < pending; t0 += 2) {  // (rows past the pending ones are zeros)
+#pragma unroll
+      for (uint32_t t = t0; t < t0 + 2; ++t) {
+        const float u0 = sh.u[t][srow], u1 = sh.u[t][srow + 8];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 k2 = *reinterpret_cast<const float2 *>(&sh.pk[t][scol + 16 * (c >> 1) + 8 * (c & 1)]);
+          const int at = 8 * (c >> 1) + 2 * (c & 1);
+          S[at] = fmaf(u0, k2.x, S[at]), S[at + 1] = fmaf(u0, k2.y, S[at + 1]);
+          S[at + 4] = fmaf(u1, k2.x, S[at + 4]), S[at + 5] = fmaf(u1, k2.y, S[at + 5]);
         }
-        o_s[t][srow] = res;
       }
     }
   }
-  __syncthreads();
-  // recurrent outputs (bf16) of this CTA's value dimensions -> scratch
-  for (uint32_t i = tid; i < rows * kGdnVd; i += kGdnThreads)
-    p.scratch[(size_t(h) * kGdnRows + i / kGdnVd) * kD + vd0 + i % kGdnVd] = float_to_bf16_bits(o_s[i / kGdnVd][i % kGdnVd]);
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) s_last = atomicAdd(&p.counters[h], 1u) == kGdnSplit - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  // (5) gated RMSNorm: a warp per row, dimensions 32 g + lane, the four partial sums added in order.
-  const uint32_t out_head = a.tiled ? (h % per_key) * KH + h / per_key : h;
-  for (uint32_t r = warp; r < rows; r += kGdnThreads / 32) {
-    float val[4], total = 0.0f;
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      val[g] = bf16_bits_to_float(__ldcg(p.scratch + (size_t(h) * kGdnRows + r) * kD + 32 * g + lane));
-      total += warp_sum(val[g] * val[g]);
-    }
-    const float inv = rsqrtf(total / float(kD) + 1e-6f);
+  for (int b = 0; b < 2; ++b)
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      const uint32_t d = 32 * g + lane;
-      const float normalized = round_bf16((val[g] * inv) * a.norm_w[d]);
-      const float z = bf16_bits_to_float(qkvz[size_t(r) * a.qkvz_stride + C + h * kD + d]);
-      static_cast<uint16_t *>(a.hidden)[size_t(r) * a.hidden_stride + out_head * kD + d] =
-          float_to_bf16_bits((normalized * z) / (1.0f + exp2f(-1.44269504089f * z)));
-    }
+    for (int second = 0; second < 2; ++second)
+#pragma unroll
+      for (int pair = 0; pair < 2; ++pair)
+        *reinterpret_cast<float2 *>(a.state_out + sbase + size_t(8 * second) * kD + 16 * b + 8 * pair) =
+            make_float2(S[8 * b + 4 * second + 2 * pair], S[8 * b + 4 * second + 2 * pair + 1]);
+  // (4) the rows' inner products (this CTA: rows vs, vs + 4, ..), and S k_t, S q_t on the tensor cores: the state as three bf16
+  // terms, k and q are bf16 as they stand, so every product is exact; the small terms first, a quarter of the columns a warp,
+  // the quarters added in fp32.
+  {
+    const uint32_t t = 4 * (warp >> 1) + vs;
+    auto key = [&](int j) { return block_row(0, j); };
+    if (t < rows) inner_products(key, block_row(warp & 1, t), (warp & 1) ? sh.kq : sh.kk, t);
   }
-  if (tid == 0) p.counters[h] = 0;
+  cluster_arrive();  // (3)
+  {
+    float acc[4][4] = {};
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      uint32_t hi[4], mid[4], lo[4];  // A: (row, pair), (row + 8, pair), (row, second pair), (row + 8, second pair)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int at = 8 * b + 4 * (i & 1) + 2 * (i >> 1);
+        split3(S[at], S[at + 1], hi[i], mid[i], lo[i]);
+      }
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {  // k rows 0-7, 8-15, q rows 0-7, 8-15
+        const uint16_t *x = &sh.x[n >> 1][8 * (n & 1) + g4][scol + 16 * b];
+        const uint32_t b0 = *reinterpret_cast<const uint32_t *>(x), b1 = *reinterpret_cast<const uint32_t *>(x + 8);
+        mma_bf16(acc[n], lo[0], lo[1], lo[2], lo[3], b0, b1);
+        mma_bf16(acc[n], mid[0], mid[1], mid[2], mid[3], b0, b1);
+        mma_bf16(acc[n], hi[0], hi[1], hi[2], hi[3], b0, b1);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sh.part[quarter][8 * n + 2 * t4 + (i & 1)][srow + 8 * (i >> 1)] = acc[n][i];
+  }
+  if (qk_writer)
+    for (uint32_t i = tid; i < rows * kD / 2; i += kGdnThreads)
+      store_pair(static_cast<uint16_t *>(a.step.k) + size_t(i / (kD / 2)) * KW + kh * kD + 2 * (i % (kD / 2)),
+                 *reinterpret_cast<const uint32_t *>(&sh.x[0][i / (kD / 2)][2 * (i % (kD / 2))]));
+  // what the gate of the row this warp will finish reads
+  const uint32_t out_row = 4 * vs + warp;
+  const bool finishes = warp < kGdnRows / kGdnSplit && out_row < rows;
+  float z[4], nw[4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    z[g] = finishes ? bf16_bits_to_float(qkvz[size_t(out_row) * a.qkvz_stride + C + h * kD + 32 * g + lane]) : 0.0f;
+    nw[g] = finishes ? a.norm_w[32 * g + lane] : 0.0f;
+  }
+  cluster_wait();   // (3) the inner products
+  __syncthreads();  // this CTA's products (written since it arrived)
+  {
+    // Coefficients of the system ([j][t], into the pending rows' matrix) and of the outputs ([t][j]): G(t, j) along row t's path, j
+    // on it; D_t (S k_t) and the outputs' first terms. Rows past the block are zeros.
+    const bool there = ct < rows, on = there && cj <= ct && (sh.path[ct] >> cj & 1u);
+    const uint32_t path = there ? sh.path[ct] : 0u;
+    const float g = decays(sh.decay, path & ~((2u << cj) - 1u)), d = decays(sh.decay, path);
+    sh.pkk[cj][ct] = on && cj < ct ? g * sh.kk[ct][cj] : 0.0f;
+    sh.kq[ct][cj] = on ? g * sh.kq[ct][cj] : 0.0f;
+    float2 right = make_float2(0.0f, 0.0f), first = right;
+    if (there) {
+      const float2 sk = four(sh.part, ct), sq = four(sh.part, kGdnRows + ct);
+      right = make_float2(d * sk.x, d * sk.y);
+      first = make_float2(d * sq.x, d * sq.y);
+    }
+    *reinterpret_cast<float2 *>(&sh.u[ct][cv]) = right;
+    *reinterpret_cast<float2 *>(&sh.o[ct][cv]) = first;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    float u[kGdnRows];
+    solve(sh.pkk, sh.v, sh.beta, u);
+#pragma unroll
+    for (int t = 0; t < kGdnRows; ++t) sh.u[t][lane] = u[t];
+  }
+  __syncthreads();
+  for (uint32_t t = warp; t < rows; t += kGdnThreads / 32) {
+    float o = sh.o[t][lane];
+#pragma unroll
+    for (int j4 = 0; j4 < kGdnRows; j4 += 4) {  // (coefficients past t are zeros)
+      if (uint32_t(j4) > t) break;
+      const float4 c4 = *reinterpret_cast<const float4 *>(&sh.kq[t][j4]);
+      o = fmaf(c4.x, sh.u[j4][lane], o), o = fmaf(c4.y, sh.u[j4 + 1][lane], o);
+      o = fmaf(c4.z, sh.u[j4 + 2][lane], o), o = fmaf(c4.w, sh.u[j4 + 3][lane], o);
+    }
+    head_ctas.map_shared_rank(&sh.out[t % 4][vd0 + lane], int(t / 4))[0] = round_bf16(o);
+  }
+  head_ctas.sync();  // (4) this CTA's rows, all 128 value dimensions
+  // (5) gated RMSNorm: a warp per row, dimensions 32 g + lane, the four partial sums added in order.
+  if (!finishes) return;
+  const uint32_t out_head = a.tiled ? (h % per_key) * KH + h / per_key : h;
+  float val[4], total = 0.0f;
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    val[g] = sh.out[warp][32 * g + lane];
+    total += warp_sum(val[g] * val[g]);
+  }
+  const float inv = rsqrtf(total / float(kD) + 1e-6f);
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const uint32_t d = 32 * g + lane;
+    const float normalized = round_bf16((val[g] * inv) * nw[g]);
+    static_cast<uint16_t *>(a.hidden)[size_t(out_row) * a.hidden_stride + out_head * kD + d] =
+        float_to_bf16_bits((normalized * z[g]) / (1.0f + exp2f(-1.44269504089f * z[g])));
+  }
 }
-
 
 // Whether the call needs the tree kernel: tree rows, or a pending path that is not known here to be the tape's first rows.
 static bool needs_tree_kernel(const SbGdnArgs &a) {
   return a.tree || a.pending_path_dev || (a.pending_path & (a.pending_path + 1u)) != 0;
 }
 
-// ---- the same step with no allocation anywhere ----
-// Some hosts of this library may not allocate device memory at all once they are running: a runtime that
-// reserved the whole GPU for its own arena up front, a plugin loaded into such a process, or code that runs
-// where cudaMalloc would fail or stall (inside a memory-pool callback, under a fixed memory budget). The
-// regular entry point uses two pieces of scratch that sb_init allocated: the recurrent rows awaiting their
-// gate and one arrival counter per value head. This variant keeps both in a fixed array that is part of the
-// library image, so every GPU that loads the library holds kStaticScratchBytes of it until the process exits.
+// The limit of sb_gdn_verify_static (its scratch once held this many heads; the kernel needs none now).
 constexpr uint32_t kStaticMaxValueHeads = 64;  // the 27B shape has 48
-constexpr size_t kStaticRowsBytes = size_t(kStaticMaxValueHeads) * kGdnRows * kD * sizeof(uint16_t);  // 256 KiB
-constexpr size_t kStaticScratchBytes = kStaticRowsBytes + kStaticMaxValueHeads * sizeof(uint32_t);
-static __device__ __align__(256) uint8_t g_gdn_static_scratch[kStaticScratchBytes];
-
-// In host code the array's name only stands for the symbol; the address a kernel can use comes from
-// cudaGetSymbolAddress, asked once per device with that device current.
-static int static_scratch_address(uint8_t **out) {
-  constexpr int kMaxDevices = 64;
-  static std::atomic<uint8_t *> address[kMaxDevices];  // (two threads racing here store the same value)
-  int device = -1;
-  SB_CUDA(cudaGetDevice(&device));
-  SB_REQUIRE(device >= 0 && device < kMaxDevices, "sb_gdn_verify_static: device index %d outside 0..%d", device, kMaxDevices - 1);
-  if (!address[device].load(std::memory_order_acquire)) {
-    void *p = nullptr;
-    SB_CUDA(cudaGetSymbolAddress(&p, g_gdn_static_scratch));
-    SB_REQUIRE(p != nullptr, "sb_gdn_verify_static: the scratch symbol has no address on device %d", device);
-    address[device].store(static_cast<uint8_t *>(p), std::memory_order_release);
-  }
-  *out = address[device].load(std::memory_order_acquire);
-  return SB_OK;
-}
 
 }  // namespace sb
 
@@ -506,52 +684,44 @@ static int gdn_validate(const SbGdnArgs *a, const char *who) {
                                  (reinterpret_cast<uintptr_t>(a->gate_weight) & 15) == 0 && (reinterpret_cast<uintptr_t>(a->gate_input) & 15) == 0),
              "%s: fused gate projection needs a 16-byte aligned input and weight, k a multiple of 8 and stride >= k", who);
   SB_REQUIRE((a->flags & ~uint32_t(SB_GDN_STATE_SETTLED)) == 0, "%s: unknown flags 0x%x", who, a->flags);
-  SB_REQUIRE(a->lanes <= 64 && size_t(std::max(1u, a->lanes)) * a->value_heads <= kGdnScratchHeads, "%s: %u lanes of %u value heads exceed the scratch", who,
+  SB_REQUIRE(a->lanes <= 64 && size_t(std::max(1u, a->lanes)) * a->value_heads <= kGdnLaunchHeads, "%s: %u lanes of %u value heads exceed a launch", who,
              a->lanes, a->value_heads);
   return SB_OK;
 }
 }  // namespace sb
 
-extern "C" int sb_gdn_verify(void *stream, const SbGdnArgs *a) {
-  SB_NEED_DEVICE();
-  const int valid = gdn_validate(a, "sb_gdn_verify");
-  if (valid != SB_OK) return valid;
-  Context &c = ctx();
-  GdnParams p{*a, c.gdn_scratch, c.gdn_counters};
+static int gdn_launch(void *stream, const SbGdnArgs *a, bool pdl) {
+  const GdnParams p{*a};
+  const bool tree = needs_tree_kernel(*a), several = a->lanes > 1;
+  const auto kernel = several ? (tree ? gdn_kernel<true, 4> : gdn_kernel<false, 4>) : (tree ? gdn_kernel<true, 2> : gdn_kernel<false, 2>);
+  static std::atomic<uint64_t> allowed[4];
+  const int st = allow_smem(reinterpret_cast<const void *>(kernel), sizeof(GdnShared), allowed[2 * several + tree]);
+  if (st != SB_OK) return st;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kGdnSplit, a->value_heads, std::max(1u, a->lanes));
   cfg.blockDim = dim3(kGdnThreads);
+  cfg.dynamicSmemBytes = sizeof(GdnShared);
   cfg.stream = as_stream(stream);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = c.pdl ? 1 : 0;
-  if (a->lanes > 1)
-    SB_CUDA(needs_tree_kernel(*a) ? cudaLaunchKernelEx(&cfg, gdn_kernel<true, 4>, p) : cudaLaunchKernelEx(&cfg, gdn_kernel<false, 4>, p));
-  else
-    SB_CUDA(needs_tree_kernel(*a) ? cudaLaunchKernelEx(&cfg, gdn_kernel<true>, p) : cudaLaunchKernelEx(&cfg, gdn_kernel<false>, p));
+  cfg.numAttrs = pdl ? 1 : 0;
+  SB_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
   return SB_OK;
+}
+
+extern "C" int sb_gdn_verify(void *stream, const SbGdnArgs *a) {
+  SB_NEED_DEVICE();
+  const int valid = gdn_validate(a, "sb_gdn_verify");
+  return valid != SB_OK ? valid : gdn_launch(stream, a, ctx().pdl);
 }
 
 extern "C" int sb_gdn_verify_static(void *stream, const SbGdnArgs *a) {
   SB_REQUIRE(a, "sb_gdn_verify_static: null arguments");
-  SB_REQUIRE(a->value_heads <= kStaticMaxValueHeads,
-             "sb_gdn_verify_static: %u value heads exceed the %u the built-in scratch holds; use sb_gdn_verify", a->value_heads,
+  SB_REQUIRE(a->value_heads <= kStaticMaxValueHeads, "sb_gdn_verify_static: %u value heads exceed %u; use sb_gdn_verify", a->value_heads,
              kStaticMaxValueHeads);
-  SB_REQUIRE(a->lanes <= 1, "sb_gdn_verify_static: one lane a call (the built-in scratch holds one lane's rows)");
+  SB_REQUIRE(a->lanes <= 1, "sb_gdn_verify_static: one lane a call");
   const int valid = gdn_validate(a, "sb_gdn_verify_static");
-  if (valid != SB_OK) return valid;
-  uint8_t *scratch = nullptr;
-  const int st = static_scratch_address(&scratch);
-  if (st != SB_OK) return st;
-  // The array keeps whatever the last call left. The arrival counters must start at zero; the rows are
-  // written in full before they are read.
-  uint32_t *counters = reinterpret_cast<uint32_t *>(scratch + kStaticRowsBytes);
-  SB_CUDA(cudaMemsetAsync(counters, 0, kStaticMaxValueHeads * sizeof(uint32_t), as_stream(stream)));
-  GdnParams p{*a, reinterpret_cast<uint16_t *>(scratch), counters};
-  if (needs_tree_kernel(*a)) gdn_kernel<true><<<dim3(kGdnSplit, a->value_heads), dim3(kGdnThreads), 0, as_stream(stream)>>>(p);
-  else gdn_kernel<false><<<dim3(kGdnSplit, a->value_heads), dim3(kGdnThreads), 0, as_stream(stream)>>>(p);
-  SB_CUDA(cudaGetLastError());
-  return SB_OK;
+  return valid != SB_OK ? valid : gdn_launch(stream, a, false);
 }

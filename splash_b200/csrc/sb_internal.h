@@ -4,6 +4,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "../../include/splash_b200.h"
 
 namespace sb {
@@ -24,8 +26,6 @@ struct Context {
   float *attn_workspace = nullptr;       // split partials and (max, sum) of sb_attn_verify
   size_t attn_workspace_bytes = 0;
   uint32_t *attn_counters = nullptr;     // one arrival counter per KV head, zero between launches
-  uint16_t *gdn_scratch = nullptr;       // recurrent outputs before the gate [value_heads][16][128]
-  uint32_t *gdn_counters = nullptr;      // one arrival counter per value head
   bool pdl = true;                       // launch glue kernels with programmatic stream serialization
   int tp_exchange_shots = 0;             // 0: by the number of ranks, 1: one shot, 2: two shots (sb_tp_set_exchange)
   uint64_t wait_ns = 2000000000ull;      // how long a kernel waits for a peer GPU before it gives up (sb_set_wait_limit_ns)
@@ -53,7 +53,7 @@ int cuda_fail(cudaError_t e, const char *what);
   } while (0)
 
 constexpr uint32_t kAttnCounterWords = 64 * 128;  // 128 arrival / merge counters per lane, up to 64 lanes
-constexpr uint32_t kGdnScratchHeads = 2048;       // value heads x lanes of one sb_gdn_verify launch
+constexpr uint32_t kGdnLaunchHeads = 2048;        // value heads x lanes of one sb_gdn_verify launch
 
 // Device status word values.
 enum : uint32_t {
@@ -61,6 +61,18 @@ enum : uint32_t {
   SB_DEV_WAIT_EXPIRED = 1,  // a bounded mbarrier / flag wait gave up
   SB_DEV_CONTRACT = 2       // a kernel met arguments outside its contract and returned early
 };
+
+// Lets `kernel` have `bytes` of dynamic shared memory on the current device; the attribute stays with the function, so it is set
+// at the kernel's first launch on a device only (`done`: a bit a device, the kernel's own).
+inline int allow_smem(const void *kernel, size_t bytes, std::atomic<uint64_t> &done) {
+  int device = 0;
+  SB_CUDA(cudaGetDevice(&device));
+  const uint64_t bit = uint64_t(1) << (device & 63);
+  if (done.load(std::memory_order_acquire) & bit) return SB_OK;
+  SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  done.fetch_or(bit, std::memory_order_release);
+  return SB_OK;
+}
 
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 

@@ -776,7 +776,11 @@ template <class A> static int launch_selection(void (*cluster)(A), void (*block)
   attr[1].val.clusterDim.x = kSelectCtas, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = clusters ? 2 : 1;
-  if (clusters) SB_CUDA(cudaFuncSetAttribute(cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, int(select_smem_bytes(kSelectVocab))));
+  if (clusters) {
+    static std::atomic<uint64_t> allowed;  // (one a kind of arguments, that is, one a kernel)
+    const int st = allow_smem(reinterpret_cast<const void *>(cluster), select_smem_bytes(kSelectVocab), allowed);
+    if (st != SB_OK) return st;
+  }
   SB_CUDA(cudaLaunchKernelEx(&cfg, clusters ? cluster : block, args));
   return SB_OK;
 }

@@ -6,130 +6,270 @@
 //   intermediate = bf16(bf16(up . x) * silu(bf16(gate . x)))     per route
 //   y            = bf16(down . intermediate)                     per route
 //   out          = bf16(residual + sum over the row's routes, in slot order, of weight * float(y))
-// The reference groups routes by expert into tiles so that an expert's weights stream once for many rows; with at
-// most 16 rows nearly every route has its expert to itself, so a route streams its expert's rows directly: a warp per
-// output column, a lane per 8 consecutive weights of every super-block, effective weights d sc q - dmin m unrounded
-// (as in linear_kernel), fp32 sums. The grouped tile kernel for the M >= 64 regime is not built.
+// The routes are grouped by expert (up to eight a group, the columns of one MMA), so an expert's weights are read once for all the
+// rows that chose it. A matrix-vector product a route (the first form) spent some 3 instructions a weight and route: 186 us for 16
+// rows of the 35B-A3B shape, 1.0 TB/s. Now a warp takes 16 gate and the 16 up rows (32 down rows) of a group over the whole of K:
+// lane 4 g + t loads rows g and g + 8's sub-blocks 2t, 2t + 1 of every super-block straight into registers (two 16-byte loads a row
+// and a header) and feeds them to mma.sync as exact integers sc q (sb_q4k.cuh) against the group's activations in fp16, exact too
+// (a power of two a row), the block scales on fp32 sums: 76 us for the same 16 rows, 180 MB of experts' weights in some 62 us of two
+// expert passes (2.6 TB/s). What bounds them is the L1: a warp's 16-byte loads touch eight rows each, and the activations come the
+// same way. Tried: the next unit's rows prefetched into the L2 (84 us), three CTAs a SM at 80 registers (78 us).
 #include <algorithm>
 
 #include "sb_internal.h"
 #include "sb_linear_internal.h"
 #include "sb_ptx.cuh"
+#include "sb_q4k.cuh"
 
 namespace sb {
 
+constexpr uint32_t kMoeFewRows = 16, kMoeFewRoutes = kMoeFewRows * 32;  // rows and routes of a lane's block
 constexpr int kMoeThreads = 256, kMoeWarps = kMoeThreads / 32;
-constexpr int kMoeColsPair = 8, kMoeColsDown = 8;  // output columns a warp computes against the staged row (gate/up pass, down pass)
 
-// scale and min of sub-block j of a Q4_K super-block from its 12 packed bytes (three words), in registers: bytes 0-3
-// hold the low 6 bits of scales 0-3 (and in their top 2 bits the high bits of scales 4-7), bytes 4-7 the same for the mins,
-// bytes 8-11 the low nibbles of scales 4-7 (low half) and mins 4-7 (high half).
-__device__ __forceinline__ void q4k_scale_min(const uint32_t (&w)[3], uint32_t j, float &sc, float &mn) {
-  const uint32_t s8 = 8 * (j & 3);
-  uint32_t isc, imn;
-  if (j < 4) {
-    isc = (w[0] >> s8) & 63u, imn = (w[1] >> s8) & 63u;
-  } else {
-    isc = ((w[2] >> s8) & 0xFu) | (((w[0] >> (s8 + 6)) & 3u) << 4);
-    imn = ((w[2] >> (s8 + 4)) & 0xFu) | (((w[1] >> (s8 + 6)) & 3u) << 4);
-  }
-  sc = float(isc), mn = float(imn);
-}
-
-// acc[m][c] += lane's share of dot(row c of matrix m, x) for NC consecutive Q4_K rows of each of NM matrices; x staged in
-// shared memory as floats; lane l takes weights 32 (l / 4) + 8 (l % 4) .. + 7 of every super-block, so the lane's x values
-// and their sum are fetched once per super-block for all the rows.
-template <int NM, int NC>
-__device__ __forceinline__ void q4k_rows_dot(const uint8_t *const (&rows)[NM], size_t row_bytes, const float *x, uint32_t k, uint32_t lane,
-                                             float (&acc)[NM][NC]) {
-  const uint32_t sub = lane >> 2, t0 = 8 * (lane & 3), shift = (sub & 1) * 4;
-#pragma unroll
-  for (int m = 0; m < NM; ++m)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) acc[m][c] = 0.0f;
-#pragma unroll 2
-  for (uint32_t sb = 0; sb < k / 256; ++sb) {
-    const float4 x0 = *reinterpret_cast<const float4 *>(x + 256 * sb + 32 * sub + t0), x1 = *reinterpret_cast<const float4 *>(x + 256 * sb + 32 * sub + t0 + 4);
-    const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-    const float xsum = ((xs[0] + xs[1]) + (xs[2] + xs[3])) + ((xs[4] + xs[5]) + (xs[6] + xs[7]));
-#pragma unroll
-    for (int m = 0; m < NM; ++m)
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const uint8_t *blk = rows[m] + size_t(c) * row_bytes + size_t(sb) * 144;
-        const uint32_t dm = *reinterpret_cast<const uint32_t *>(blk);
-        const float d = __half2float(__ushort_as_half(uint16_t(dm & 0xffffu))), dmin = __half2float(__ushort_as_half(uint16_t(dm >> 16)));
-        const uint32_t sw[3] = {*reinterpret_cast<const uint32_t *>(blk + 4), *reinterpret_cast<const uint32_t *>(blk + 8),
-                                *reinterpret_cast<const uint32_t *>(blk + 12)};
-        float sc, mn;
-        q4k_scale_min(sw, sub, sc, mn);
-        const uint2 qs = *reinterpret_cast<const uint2 *>(blk + 16 + 32 * (sub >> 1) + t0);
-        float qx = 0.0f;
-        const uint32_t n0 = (qs.x >> shift) & 0x0F0F0F0Fu, n1 = (qs.y >> shift) & 0x0F0F0F0Fu;  // the lane's eight codes, a byte each
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          // the code as a float without a conversion instruction (quarter rate): 2^23 + q in the mantissa, minus 2^23
-          const float q = __uint_as_float(0x4B000000u | __byte_perm(j < 4 ? n0 : n1, 0, 0x4440 + (j & 3))) - 8388608.0f;
-          qx = fmaf(q, xs[j], qx);
-        }
-        acc[m][c] = fmaf(d * sc, qx, acc[m][c]);
-        acc[m][c] = fmaf(-dmin * mn, xsum, acc[m][c]);
-      }
-  }
-#pragma unroll
-  for (int m = 0; m < NM; ++m)
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-      for (int o = 16; o; o >>= 1) acc[m][c] += __shfl_xor_sync(0xffffffffu, acc[m][c], o);
+// Up to eight routes of one expert.
+struct MoeFew {
+  uint32_t expert, n, route[8];
+};
+// The scratch of a call: activations as the expert kernels read them, the intermediate rows, the routes' results, the groups.
+struct MoeFewLayout {
+  uint64_t counts, groups, x, x_scale, act, act_scale, intermediate, y, bytes;
+};
+// A converted row of k inputs: per super-block 512 bytes of 16-byte units, then per super-block 32 bytes of sub-block sums.
+__host__ __device__ inline uint64_t moe_row_bytes(uint32_t k) { return uint64_t(k) * 2 + k / 8; }
+static MoeFewLayout moe_few_layout(uint32_t rows, uint32_t routes, uint32_t hidden, uint32_t inter) {
+  MoeFewLayout l{};
+  const uint64_t n = uint64_t(rows) * routes;
+  uint64_t at = 0;
+  auto take = [&](uint64_t bytes) { const uint64_t here = at; at += (bytes + 255) / 256 * 256; return here; };
+  l.intermediate = take(n * inter * 2), l.y = take(n * hidden * 2);
+  l.counts = take(4), l.groups = take(n * sizeof(MoeFew)), l.x = take(rows * moe_row_bytes(hidden)), l.x_scale = take(rows * 4);
+  l.act = take(n * moe_row_bytes(inter)), l.act_scale = take(n * 4);
+  l.bytes = at;
+  return l;
 }
 
 struct MoeParams {
   SbMoeExpertArgs a;
   uint16_t *intermediate;  // bf16 [rows * routes, inter]
   uint16_t *y;             // bf16 [rows * routes, hidden]
+  uint32_t *counts;        // [0] groups
+  MoeFew *groups;
+  uint8_t *x, *act;         // converted rows: [rows], [rows * routes]
+  float *x_scale, *act_scale;
 };
 
-// PAIR: gate and up of the route's expert over the row's input -> intermediate. Otherwise: down over the route's
-// intermediate -> y. grid (rows * routes, column blocks).
-template <bool PAIR> __global__ void __launch_bounds__(kMoeThreads) moe_expert_kernel(const MoeParams p) {
-  constexpr int kMoeColsPerWarp = PAIR ? kMoeColsPair : kMoeColsDown;
-  extern __shared__ float xrow[];
+// A bf16 row in fp16 with a power of two taken out (exact for values down to 2^-24 of the row's largest), in the order a lane of
+// the expert kernels reads it: unit (i2, p, t) of a super-block holds inputs 32 (2 t + p) + 8 i2 .. + 7 as [0,2,1,3,4,6,5,7] (the
+// order the Q4_K nibbles come out in), and lane t's 8 bytes of sums are sub-blocks 2 t, 2 t + 1, each a high and a low half.
+__device__ __forceinline__ void moe_convert_row(const uint16_t *src, uint32_t k, uint8_t *dst, float *scale, float *scratch) {
+  const uint32_t tid = threadIdx.x, chunks = k / 8;
+  const bool wide = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  constexpr int kMost = 8192 / 8 / kMoeThreads;  // chunks a thread keeps
+  float v[kMost][8], mx = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kMost; ++i) {
+    const uint32_t c = tid + i * blockDim.x;
+    uint32_t u[4] = {0, 0, 0, 0};
+    if (c < chunks) {
+      if (wide) {
+        const uint4 w = *reinterpret_cast<const uint4 *>(src + 8 * c);
+        u[0] = w.x, u[1] = w.y, u[2] = w.z, u[3] = w.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) u[j] = uint32_t(src[8 * c + 2 * j]) | (uint32_t(src[8 * c + 2 * j + 1]) << 16);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[i][2 * j] = bf16_bits_to_float(u[j] & 0xffffu), v[i][2 * j + 1] = bf16_bits_to_float(u[j] >> 16);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(v[i][j]));  // (NaN does not win a max; it stays in the values)
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((tid & 31) == 0) scratch[tid >> 5] = mx;
+  __syncthreads();
+  for (uint32_t w = 0; w < blockDim.x / 32; ++w) mx = fmaxf(mx, scratch[w]);
+  int e = 0;
+  if (mx > 0.0f && mx <= 3.0e38f) {
+    (void)frexpf(mx, &e);
+    e -= 10;  // scaled values stay below 2^10
+  }
+  const float down = ldexpf(1.0f, -e);
+  if (tid == 0) *scale = ldexpf(1.0f, e);
+#pragma unroll
+  for (int i = 0; i < kMost; ++i) {
+    const uint32_t c = tid + i * blockDim.x;
+    if (c >= chunks) break;  // (whole warps: chunks is a multiple of 32)
+    const uint32_t sb = c >> 5, j = (c & 31u) >> 2, q = c & 3u;
+    __half h[8];
+    float sum = 0.0f;
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj) h[jj] = __float2half_rn(v[i][jj] * down), sum += __half2float(h[jj]);
+    const __half2 p0 = __halves2half2(h[0], h[2]), p1 = __halves2half2(h[1], h[3]), p2 = __halves2half2(h[4], h[6]), p3 = __halves2half2(h[5], h[7]);
+    *reinterpret_cast<uint4 *>(dst + size_t(sb) * 512 + ((q * 2 + (j & 1)) * 4 + (j >> 1)) * 16) =
+        make_uint4(*reinterpret_cast<const uint32_t *>(&p0), *reinterpret_cast<const uint32_t *>(&p1), *reinterpret_cast<const uint32_t *>(&p2),
+                   *reinterpret_cast<const uint32_t *>(&p3));
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);  // 32 inputs = 4 consecutive lanes
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (q == 0) {
+      const __half hi = __float2half_rn(sum), lo = __float2half_rn(sum - __half2float(hi));
+      *reinterpret_cast<__half2 *>(dst + size_t(k) * 2 + size_t(sb) * 32 + j * 4) = __halves2half2(hi, lo);
+    }
+  }
+}
+
+// grid (rows + 1): a CTA a row of the input, and one that groups the routes. A route's place among its expert's routes is the
+// number of earlier routes of the expert; every eighth of them starts a group, groups in the order they start.
+__global__ void __launch_bounds__(kMoeThreads) moe_few_prepare_kernel(const MoeParams p) {
+  __shared__ float scratch[kMoeWarps];
+  __shared__ uint32_t expert_s[kMoeFewRoutes], rank_s[kMoeFewRoutes], group_s[kMoeFewRoutes], warp_s[2 * kMoeWarps];
   pdl_launch_dependents();
   pdl_wait();
   const SbMoeExpertArgs &a = p.a;
-  const uint32_t route = blockIdx.x, row = route / a.routes, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t k = PAIR ? a.hidden : a.inter, n = PAIR ? a.inter : a.hidden;
-  const uint32_t expert = min(a.selected[route], a.experts_total - 1);
-  const uint16_t *src = PAIR ? static_cast<const uint16_t *>(a.input) + size_t(row) * a.hidden : p.intermediate + size_t(route) * a.inter;
-  for (uint32_t i = tid; i < k; i += kMoeThreads) xrow[i] = bf16_bits_to_float(src[i]);
+  if (blockIdx.x < a.rows) {
+    const uint32_t row = blockIdx.x;
+    moe_convert_row(static_cast<const uint16_t *>(a.input) + size_t(row) * a.hidden, a.hidden, p.x + row * moe_row_bytes(a.hidden), p.x_scale + row, scratch);
+    return;
+  }
+  const uint32_t n = a.rows * a.routes, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (uint32_t i = tid; i < n; i += kMoeThreads) expert_s[i] = min(a.selected[i], a.experts_total - 1);
   __syncthreads();
-  const size_t row_bytes = size_t(k / 256) * 144;
-  const uint8_t *w0 = static_cast<const uint8_t *>(PAIR ? a.gate : a.down) + size_t(expert) * n * row_bytes;
-  const uint8_t *w1 = PAIR ? static_cast<const uint8_t *>(a.up) + size_t(expert) * n * row_bytes : nullptr;
-  const uint32_t c0 = (blockIdx.y * kMoeWarps + warp) * kMoeColsPerWarp;
-  if (c0 >= n) return;  // n is a multiple of 256, so a warp's columns are inside or outside together
-  if (PAIR) {
-    const uint8_t *const rows[2] = {w0 + size_t(c0) * row_bytes, w1 + size_t(c0) * row_bytes};
-    float acc[2][kMoeColsPerWarp];
-    q4k_rows_dot<2, kMoeColsPerWarp>(rows, row_bytes, xrow, k, lane, acc);
-    if (lane < kMoeColsPerWarp) {
-      float g = 0.0f, u = 0.0f;
+  // thread t: routes t and t + 256, numbered in that order by warp and lane
+  uint32_t rank[2], starts[2];
 #pragma unroll
-      for (int c = 0; c < kMoeColsPerWarp; ++c)
-        if (lane == uint32_t(c)) g = acc[0][c], u = acc[1][c];
-      p.intermediate[size_t(route) * a.inter + c0 + lane] = float_to_bf16_bits(round_bf16(u) * silu_f(round_bf16(g)));
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t i = tid + k * kMoeThreads;
+    rank[k] = 0;
+    if (i < n)
+      for (uint32_t j = 0; j < i; ++j) rank[k] += expert_s[j] == expert_s[i];
+    if (i < n) rank_s[i] = rank[k];
+    starts[k] = __ballot_sync(0xffffffffu, i < n && (rank[k] & 7u) == 0);
+    if (lane == 0) warp_s[k * kMoeWarps + warp] = uint32_t(__popc(starts[k]));
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t i = tid + k * kMoeThreads;
+    uint32_t before = 0;
+    for (int w = 0; w < k * kMoeWarps + int(warp); ++w) before += warp_s[w];
+    if (i < n && (rank[k] & 7u) == 0) group_s[i] = before + uint32_t(__popc(starts[k] & ((1u << lane) - 1u)));
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t i = tid + k * kMoeThreads;
+    if (i >= n) break;
+    const uint32_t e = expert_s[i], first = rank[k] & ~7u;
+    uint32_t start = i, total = 0;
+    for (uint32_t j = 0; j < n; ++j)
+      if (expert_s[j] == e) {
+        ++total;
+        if (rank_s[j] == first) start = j;
+      }
+    MoeFew &g = p.groups[group_s[start]];
+    g.route[rank[k] & 7u] = i;
+    if (start == i) g.expert = e, g.n = min(total - first, 8u);
+  }
+  if (tid == 0) {
+    uint32_t groups = 0;
+    for (int w = 0; w < 2 * kMoeWarps; ++w) groups += warp_s[w];
+    p.counts[0] = groups;
+  }
+}
+
+// grid (rows * routes): a route's intermediate row.
+__global__ void __launch_bounds__(kMoeThreads) moe_few_convert_kernel(const MoeParams p) {
+  __shared__ float scratch[kMoeWarps];
+  pdl_launch_dependents();
+  pdl_wait();
+  const uint32_t route = blockIdx.x;
+  moe_convert_row(p.intermediate + size_t(route) * p.a.inter, p.a.inter, p.act + route * moe_row_bytes(p.a.inter), p.act_scale + route, scratch);
+}
+
+// PAIR: gate and up of the groups' experts over the rows' inputs -> intermediate. Otherwise down over the routes' intermediate
+// rows -> y. A warp a (group, column block) in turn; its two 16-row tiles are the gate and the up rows of 16 columns, or the
+// down rows of 32.
+template <bool PAIR> __global__ void __launch_bounds__(kMoeThreads, 2) moe_few_kernel(const MoeParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const SbMoeExpertArgs &a = p.a;
+  const uint32_t lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t k = PAIR ? a.hidden : a.inter, n = PAIR ? a.inter : a.hidden, nsb = k / 256, blocks = n / (PAIR ? 16 : 32);
+  const size_t row_bytes = size_t(nsb) * 144, in_bytes = moe_row_bytes(k);
+  const uint32_t units = p.counts[0] * blocks, warps = gridDim.x * kMoeWarps;
+  // (neighbouring warps of a CTA on neighbouring column blocks of a group: they share its activations in the L1)
+  for (uint32_t u = blockIdx.x * kMoeWarps + (threadIdx.x >> 5); u < units; u += warps) {
+    const MoeFew &few = p.groups[u / blocks];
+    const uint32_t c0 = u % blocks * (PAIR ? 16 : 32), count = few.n;
+    const uint32_t mine = few.route[min(g, count - 1)], in_row = PAIR ? mine / a.routes : mine;  // (columns past the group repeat its last)
+    const uint8_t *in = (PAIR ? p.x : p.act) + in_row * in_bytes + t * 16, *sums = (PAIR ? p.x : p.act) + in_row * in_bytes + size_t(k) * 2 + t * 8;
+    const uint8_t *w[2];
+    w[0] = static_cast<const uint8_t *>(PAIR ? a.gate : a.down) + (size_t(few.expert) * n + c0 + g) * row_bytes;
+    w[1] = PAIR ? static_cast<const uint8_t *>(a.up) + (size_t(few.expert) * n + c0 + g) * row_bytes : w[0] + 16 * row_bytes;
+    float y[2][4] = {};
+    for (uint32_t sb = 0; sb < nsb; ++sb) {
+      uint4 hdr[2][2], q[2][2][2];
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const uint8_t *blk = w[mt] + size_t(8 * r) * row_bytes + size_t(sb) * 144;
+          hdr[mt][r] = __ldg(reinterpret_cast<const uint4 *>(blk));
+          q[mt][r][0] = __ldg(reinterpret_cast<const uint4 *>(blk + 16 + 32 * t));
+          q[mt][r][1] = __ldg(reinterpret_cast<const uint4 *>(blk + 32 + 32 * t));
+        }
+      Q4Scales sc[2][2];
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) sc[mt][r] = q4_scales(hdr[mt][r], t);
+      float aq[2][4] = {};
+      const uint32_t kMagic = 0x64006400u;
+#pragma unroll
+      for (int i2 = 0; i2 < 4; ++i2) {
+        const uint4 lo = *reinterpret_cast<const uint4 *>(in + size_t(sb) * 512 + i2 * 128), hi = *reinterpret_cast<const uint4 *>(in + size_t(sb) * 512 + i2 * 128 + 64);
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+          for (int wi = 0; wi < 2; ++wi) {
+            const uint4 q0 = q[mt][0][i2 >> 1], q1 = q[mt][1][i2 >> 1];
+            const uint32_t w0 = (i2 & 1) ? (wi ? q0.w : q0.z) : (wi ? q0.y : q0.x), w1 = (i2 & 1) ? (wi ? q1.w : q1.z) : (wi ? q1.y : q1.x);
+            const uint32_t w0s = w0 >> 8, w1s = w1 >> 8;
+            mma_f16(aq[mt], hfma2_u32(and_or(w0, 0x000f000fu, kMagic), sc[mt][0].mlo, sc[mt][0].blo),
+                    hfma2_u32(and_or(w1, 0x000f000fu, kMagic), sc[mt][1].mlo, sc[mt][1].blo),
+                    hfma2_u32(and_or(w0s, 0x000f000fu, kMagic), sc[mt][0].mlo, sc[mt][0].blo),
+                    hfma2_u32(and_or(w1s, 0x000f000fu, kMagic), sc[mt][1].mlo, sc[mt][1].blo), wi ? lo.z : lo.x, wi ? lo.w : lo.y);
+            mma_f16(aq[mt], hfma2_u32(and_or(w0, 0x00f000f0u, kMagic), sc[mt][0].mhi, sc[mt][0].bhi),
+                    hfma2_u32(and_or(w1, 0x00f000f0u, kMagic), sc[mt][1].mhi, sc[mt][1].bhi),
+                    hfma2_u32(and_or(w0s, 0x00f000f0u, kMagic), sc[mt][0].mhi, sc[mt][0].bhi),
+                    hfma2_u32(and_or(w1s, 0x00f000f0u, kMagic), sc[mt][1].mhi, sc[mt][1].bhi), wi ? hi.z : hi.x, wi ? hi.w : hi.y);
+          }
+      }
+      const uint2 s = *reinterpret_cast<const uint2 *>(sums + size_t(sb) * 32);
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt) {
+        float am[4] = {};
+        mma_f16(am, sc[mt][0].mn0, sc[mt][1].mn0, sc[mt][0].mn1, sc[mt][1].mn1, s.x, s.y);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) y[mt][c] = fmaf(sc[mt][c >> 1].ndmin, am[c], fmaf(sc[mt][c >> 1].d, aq[mt][c], y[mt][c]));
+      }
     }
-  } else {
-    const uint8_t *const rows[1] = {w0 + size_t(c0) * row_bytes};
-    float acc[1][kMoeColsPerWarp];
-    q4k_rows_dot<1, kMoeColsPerWarp>(rows, row_bytes, xrow, k, lane, acc);
-    if (lane < kMoeColsPerWarp) {
-      float v = 0.0f;
+    // lane 4 g + t: columns g and g + 8 of the group's routes 2 t, 2 t + 1
 #pragma unroll
-      for (int c = 0; c < kMoeColsPerWarp; ++c)
-        if (lane == uint32_t(c)) v = acc[0][c];
-      p.y[size_t(route) * a.hidden + c0 + lane] = float_to_bf16_bits(v);
+    for (int i = 0; i < 2; ++i) {
+      if (2 * t + i >= count) continue;
+      const uint32_t route = few.route[2 * t + i];
+      const float back = PAIR ? p.x_scale[route / a.routes] : p.act_scale[route];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const uint32_t c = c0 + g + 8 * r;
+        if (PAIR) {
+          p.intermediate[size_t(route) * a.inter + c] = float_to_bf16_bits(round_bf16(y[1][i + 2 * r] * back) * silu_f(round_bf16(y[0][i + 2 * r] * back)));
+        } else {
+          p.y[size_t(route) * a.hidden + c] = float_to_bf16_bits(y[0][i + 2 * r] * back);
+          p.y[size_t(route) * a.hidden + c + 16] = float_to_bf16_bits(y[1][i + 2 * r] * back);
+        }
+      }
     }
   }
 }
@@ -325,8 +465,7 @@ template <class K> static int launch_moe(K kernel, dim3 grid, dim3 block, size_t
 using namespace sb;
 
 extern "C" uint64_t sb_moe_scratch_bytes(uint32_t rows, uint32_t routes, uint32_t hidden, uint32_t inter) {
-  if (rows > 16) return moe_group_layout(rows, routes, hidden, inter).bytes;
-  return uint64_t(rows) * routes * (uint64_t(hidden) + inter) * 2 + 256;
+  return rows > kMoeFewRows ? moe_group_layout(rows, routes, hidden, inter).bytes : moe_few_layout(rows, routes, hidden, inter).bytes;
 }
 
 // More than 16 rows: group the routes by expert, gather and convert each group's rows, the experts' one-pass gate/up and
@@ -399,13 +538,24 @@ extern "C" int sb_moe_experts(void *stream, const SbMoeExpertArgs *a) {
   SB_NEED_DEVICE();
   const int valid = moe_check(a, "sb_moe_experts");
   if (valid != SB_OK) return valid;
-  if (a->rows > 16) return moe_experts_grouped(as_stream(stream), a);
-  MoeParams p{*a, static_cast<uint16_t *>(a->scratch), static_cast<uint16_t *>(a->scratch) + size_t(a->rows) * a->routes * a->inter};
-  const uint32_t routes = a->rows * a->routes, pair_block = kMoeWarps * kMoeColsPair, down_block = kMoeWarps * kMoeColsDown;
+  if (a->rows > kMoeFewRows) return moe_experts_grouped(as_stream(stream), a);
+  const MoeFewLayout l = moe_few_layout(a->rows, a->routes, a->hidden, a->inter);
+  uint8_t *base = static_cast<uint8_t *>(a->scratch);
+  const MoeParams p{*a,
+                    reinterpret_cast<uint16_t *>(base + l.intermediate),
+                    reinterpret_cast<uint16_t *>(base + l.y),
+                    reinterpret_cast<uint32_t *>(base + l.counts),
+                    reinterpret_cast<MoeFew *>(base + l.groups),
+                    base + l.x,
+                    base + l.act,
+                    reinterpret_cast<float *>(base + l.x_scale),
+                    reinterpret_cast<float *>(base + l.act_scale)};
   cudaStream_t s = as_stream(stream);
-  int st = launch_moe(moe_expert_kernel<true>, dim3(routes, (a->inter + pair_block - 1) / pair_block), dim3(kMoeThreads), size_t(a->hidden) * 4, s, p);
-  if (st != SB_OK) return st;
-  st = launch_moe(moe_expert_kernel<false>, dim3(routes, (a->hidden + down_block - 1) / down_block), dim3(kMoeThreads), size_t(a->inter) * 4, s, p);
+  const uint32_t routes = a->rows * a->routes, resident = uint32_t(ctx().sm_count) * 2;
+  int st = launch_moe(moe_few_prepare_kernel, dim3(a->rows + 1), dim3(kMoeThreads), 0, s, p);
+  if (st == SB_OK) st = launch_moe(moe_few_kernel<true>, dim3(resident), dim3(kMoeThreads), 0, s, p);
+  if (st == SB_OK) st = launch_moe(moe_few_convert_kernel, dim3(routes), dim3(std::min(uint32_t(kMoeThreads), a->inter / 8)), 0, s, p);
+  if (st == SB_OK) st = launch_moe(moe_few_kernel<false>, dim3(resident), dim3(kMoeThreads), 0, s, p);
   if (st != SB_OK) return st;
   return launch_moe(moe_combine_kernel, dim3((a->hidden + 255) / 256, a->rows), dim3(256), 0, s, p);
 }

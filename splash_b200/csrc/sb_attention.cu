@@ -318,10 +318,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const AttnPa
     for (int hrow = 0; hrow < 2; ++hrow) {
       const uint32_t f = warp * 16 + g + 8 * hrow;
       if (f < F) {
-        float *po = p.partials + ((size_t(kvh) * p.splits + split) * kMaxFused + f) * D;
+        float *po = p.partials + (size_t(kvh) * p.splits + split) * kMaxFused * D + 4 * f;
 #pragma unroll
-        for (int n = 0; n < NT_O; ++n)
-          *reinterpret_cast<float2 *>(po + 8 * n + 2 * t) = make_float2(o_acc[n][2 * hrow], o_acc[n][2 * hrow + 1]);
+        for (int n = 0; n < NT_O; ++n)  // dimensions 8 n + 2 t, + 1
+          *reinterpret_cast<float2 *>(po + size_t(2 * n + (t >> 1)) * 4 * kMaxFused + 2 * (t & 1)) = make_float2(o_acc[n][2 * hrow], o_acc[n][2 * hrow + 1]);
         if (t == 0) {
           float *ps = p.stats + ((size_t(kvh) * p.splits + split) * kMaxFused + f) * 2;
           ps[0] = m_run[hrow];

@@ -15,7 +15,7 @@ struct AttnParams {
   const uint2 *tree;
   uint16_t *out;
   SbKvLayer cache;
-  float *partials;     // [kv_head][split][fused][D]
+  float *partials;     // [kv_head][split][D / 4][fused][4]: rows next to each other, as both kernels write and the merge reads them
   float *stats;        // [kv_head][split][fused][2]
   uint32_t *counters;  // [kv_head] arrivals, [64 + kv_head] merges done
   uint32_t *status;
@@ -59,7 +59,7 @@ __device__ __forceinline__ void int8x16_to_half(const uint4 v, uint4 &lo, uint4 
 // The end of both kernels, called by every thread of the CTA after its split's partials (fp32 O rows and
 // (max, sum) in log2 units) are stored. Every split of this KV head publishes its partials, then all of the
 // head's CTAs (co-resident: the launch is cooperative and the grid has at most one CTA per SM) share the
-// merge: CTA `split` merges fused rows split, split + splits, ... in split order with weights
+// merge: every element's splits are added in split order with weights
 // exp2(max_s - max), divides, rounds to bf16 and multiplies by sigmoid(gate)
 // (runtime/metal/kernels/common/paged_attention_tile.h:498-535, attention_gate.h:19-45). The wait for the
 // other splits is bounded: if they never arrive the kernel sets the status word and leaves.
@@ -79,53 +79,57 @@ __device__ __forceinline__ void attention_merge(const AttnParams &p, uint32_t sp
   __syncthreads();
   if (!*s_last) return;
   __threadfence();
-  // A warp per (fused row, 128 dimensions): lane -> dimensions 128 part + 4 lane .. + 3, one 16-byte load a split, 16
-  // splits' loads in flight; the CTA's few rows so spread over all its warps. Every element is summed in split order.
-  constexpr uint32_t kParts = D / 128;
-  static_assert(D % 128 == 0, "merge tasks take 128 dimensions");
-  const uint32_t my_rows = split < F ? (F - split + p.splits - 1) / p.splits : 0;
-  for (uint32_t task = warp; task < my_rows * kParts; task += warps) {
-    const uint32_t f = split + (task / kParts) * p.splits, d0 = 128 * (task % kParts) + 4 * lane;
-    const float *stats = p.stats + (size_t(kvh) * p.splits * kMaxFused + f) * 2;
-    const float *parts = p.partials + (size_t(kvh) * p.splits * kMaxFused + f) * D + d0;
-    const size_t sstride = size_t(kMaxFused) * 2, pstride = size_t(kMaxFused) * D;
-    float mall = -INFINITY;
-    for (uint32_t s = lane; s < p.splits; s += 32) mall = fmaxf(mall, __ldcg(stats + s * sstride));
-#pragma unroll
-    for (int o = 16; o; o >>= 1) mall = fmaxf(mall, __shfl_xor_sync(0xffffffffu, mall, o));
+  // A lane per (fused row, four dimensions), neighbouring lanes neighbouring rows, so a split's share is read in runs of up to 512
+  // bytes (32 rows; 4, 8 or 16 where there are no more, and the warp's other lanes take the next dimensions); sixteen splits'
+  // loads in flight; the head's CTAs divide the tasks. Every element is summed in split order.
+  const uint32_t run = F <= 4 ? 4 : F <= 8 ? 8 : F <= 16 ? 16 : 32, row_groups = (F + run - 1) / run, tasks = D / 4 / (32 / run) * row_groups;
+  for (uint32_t task = split + p.splits * warp; task < tasks; task += p.splits * warps) {
+    const uint32_t f0 = task % row_groups * run + lane % run, f = min(f0, F - 1), d0 = (task / row_groups * (32 / run) + lane / run) * 4;
+    const bool live = f0 < F;
+    const float2 *stats = reinterpret_cast<const float2 *>(p.stats) + size_t(kvh) * p.splits * kMaxFused + f;
+    const float4 *parts = reinterpret_cast<const float4 *>(p.partials) + (size_t(kvh) * p.splits * (D / 4) + d0 / 4) * kMaxFused + f;
+    const uint32_t row = f / G, qh = kvh * G + f % G;
+    uint2 g2 = make_uint2(0, 0);
+    if (p.gated) g2 = *reinterpret_cast<const uint2 *>(p.qkv + size_t(row) * p.qkv_stride + qh * 2 * D + D + d0);
     float num[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    float den = 0.0f;
+    float den = 0.0f, m = -INFINITY;  // (the largest so far; what is summed is moved to it sixteen splits at a time)
     for (uint32_t s0 = 0; s0 < p.splits; s0 += 16) {
-      float ms[16], ls[16];
+      float2 st[16];
       float4 v[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const uint32_t s = min(s0 + j, p.splits - 1);
-        ms[j] = __ldcg(stats + s * sstride);
-        ls[j] = __ldcg(stats + s * sstride + 1);
-        v[j] = __ldcg(reinterpret_cast<const float4 *>(parts + s * pstride));
+        st[j] = make_float2(-INFINITY, 0.0f), v[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (s0 + j >= p.splits) continue;
+        st[j] = __ldcg(&stats[size_t(s0 + j) * kMaxFused]);
+        v[j] = __ldcg(parts + size_t(s0 + j) * (D / 4) * kMaxFused);
       }
+      float most = m;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) most = fmaxf(most, st[j].x);
+      if (most == -INFINITY) continue;
+      const float moved = m == -INFINITY ? 0.0f : exp2f(m - most);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) num[i] *= moved;
+      den *= moved, m = most;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        if (s0 + j >= p.splits || ms[j] == -INFINITY) continue;
-        const float w = exp2f(ms[j] - mall);
+        if (st[j].x == -INFINITY) continue;
+        const float w = exp2f(st[j].x - m);
         num[0] += w * v[j].x, num[1] += w * v[j].y, num[2] += w * v[j].z, num[3] += w * v[j].w;
-        den += w * ls[j];
+        den += w * st[j].y;
       }
     }
-    const uint32_t row = f / G, qh = kvh * G + f % G;
     float o[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[i] = round_bf16(den > 0.0f ? num[i] / den : 0.0f);
     if (p.gated) {
-      const uint2 g2 = *reinterpret_cast<const uint2 *>(p.qkv + size_t(row) * p.qkv_stride + qh * 2 * D + D + d0);
       o[0] *= sigmoid_f(bf16_bits_to_float(g2.x & 0xffffu)), o[1] *= sigmoid_f(bf16_bits_to_float(g2.x >> 16));
       o[2] *= sigmoid_f(bf16_bits_to_float(g2.y & 0xffffu)), o[3] *= sigmoid_f(bf16_bits_to_float(g2.y >> 16));
     }
     uint2 packed;
     packed.x = uint32_t(float_to_bf16_bits(o[0])) | (uint32_t(float_to_bf16_bits(o[1])) << 16);
     packed.y = uint32_t(float_to_bf16_bits(o[2])) | (uint32_t(float_to_bf16_bits(o[3])) << 16);
-    *reinterpret_cast<uint2 *>(p.out + size_t(row) * p.out_stride + qh * D + d0) = packed;
+    if (live) *reinterpret_cast<uint2 *>(p.out + size_t(row) * p.out_stride + qh * D + d0) = packed;
   }
   // The last CTA to finish its share returns both counters to zero for the next launch.
   __syncthreads();

@@ -18,6 +18,13 @@
 //             by more than 8 (p <= 256 stays far inside fp16); then the thread rescales its row of O in tensor
 //             memory once the previous chunk's P V has completed. The merge weighs splits by their own m.
 //
+// The ends of the kernel, one layer of the 27B shape at 32K with the store of its rows: 60.9 -> 53.6 us with Q turned through shared memory (a thread reading
+// its own row from memory made each load touch 32 lines: 4.9 k cycles) and the partials laid out with the rows next to each
+// other, so a split's stores and the merge's loads are up to 512 consecutive bytes (8.7 k and 12 k cycles before), read once. The loop (4.5 k
+// cycles a chunk) waits for the tensor pipe and tensor memory in turn; tried and slower: the copies issued by a warp of their own
+// (59-61 us), K and V handed over and given back separately (61 us: softmax's tensor-memory accesses take twice as long while
+// MMAs run), waits that sleep between polls (57-58 us).
+//
 // Tensor-memory columns: Q [0, D/2), S / P double buffer 2 x 64, O D columns: 512 at D = 256.
 #include <algorithm>
 
@@ -106,24 +113,45 @@ __global__ void __launch_bounds__(kAtThreads, 1) attention_tc_kernel(const AttnP
   if (warp < 4) {
     // ---- softmax warps: thread = fused row f = TMEM lane ----
     const uint32_t f = tid, tl = tmem_addr(tmem, 32 * warp, 0);
-    {  // Q row -> fp16 -> tensor memory (zeros past the fused rows)
-      const uint32_t row = f / G, hg = f % G;
-      const uint4 *src = reinterpret_cast<const uint4 *>(p.queries + (size_t(min(row, p.rows - 1)) * p.q_heads + kvh * G + hg) * D);
+    {  // Q rows -> fp16 -> tensor memory (zeros past the fused rows). A warp reads its 32 rows two at a time, 128 dimensions of each,
+       // and turns them in the second K or V buffer (chunk 1's converters wait for Q): a thread that reads its own row from memory
+       // touches 32 lines with every load of its warp.
+      constexpr uint32_t kPitch = 128 * 2;  // (16-byte units of a row exchanged by its low bits: no two of eight lanes share a bank either way)
+      static_assert(2 * 32 * kPitch <= L::kConvBytes, "two warps' rows in a buffer");
+      uint8_t *turn = smem + (warp < 2 ? L::kK : L::kV) + L::kConvBytes + (warp & 1) * 32 * kPitch;
+      
+      uint4 raw[D / 128][16];  // every load in flight at once
 #pragma unroll
-      for (int b = 0; b < D / 32; ++b) {  // 32 dimensions = 16 packed columns per store
-        uint32_t r[16];
+      for (int i = 0; i < 16; ++i) {
+        const uint32_t fr = 32 * warp + 2 * i + (lane >> 4);
+        const uint4 *src = reinterpret_cast<const uint4 *>(p.queries + (size_t(fr / G) * p.q_heads + kvh * G + fr % G) * D) + (lane & 15);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          uint4 raw = make_uint4(0, 0, 0, 0);
-          if (f < F) raw = src[4 * b + q];
-          const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+        for (int h = 0; h < D / 128; ++h) raw[h][i] = fr < F ? src[16 * h] : make_uint4(0, 0, 0, 0);
+      }
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const __half2 hv = __floats2half2_rn(bf16_bits_to_float(u[j] & 0xffffu), bf16_bits_to_float(u[j] >> 16));
-            r[4 * q + j] = *reinterpret_cast<const uint32_t *>(&hv);
-          }
+      for (int h = 0; h < D / 128; ++h) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const uint32_t r = 2 * i + (lane >> 4);
+          *reinterpret_cast<uint4 *>(turn + r * kPitch + ((lane & 15) ^ (r & 7)) * 16) = raw[h][i];
         }
-        tmem_st16(tl + 16 * b, r);
+        __syncwarp();
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {  // 32 dimensions = 16 packed columns per store
+          uint32_t r[16];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint4 w = *reinterpret_cast<const uint4 *>(turn + lane * kPitch + ((4 * b + q) ^ (lane & 7)) * 16);
+            const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const __half2 hv = __floats2half2_rn(bf16_bits_to_float(u[j] & 0xffffu), bf16_bits_to_float(u[j] >> 16));
+              r[4 * q + j] = *reinterpret_cast<const uint32_t *>(&hv);
+            }
+          }
+          tmem_st16(tl + 16 * (4 * h + b), r);
+        }
+        __syncwarp();
       }
       tmem_wait_st();
       tc_fence_before_sync();
@@ -234,7 +262,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attention_tc_kernel(const AttnP
     }
     tc_fence_after_sync();
     {
-      float *po = p.partials + ((size_t(kvh) * p.splits + split) * kMaxFused + min(f, uint32_t(kMaxFused - 1))) * D;
+      float *po = p.partials + (size_t(kvh) * p.splits + split) * kMaxFused * D + 4 * f;
 #pragma unroll 1
       for (int c0 = 0; c0 < D; c0 += 32) {
         float o[32];
@@ -243,7 +271,8 @@ __global__ void __launch_bounds__(kAtThreads, 1) attention_tc_kernel(const AttnP
         if (ok && n > 0) tmem_ld32_wait(tl + L::kOCol0 + c0, o);  // the whole warp, also lanes past the fused rows
         if (f < F)
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(po + c0 + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4 *>(po + size_t(c0 + j) * kMaxFused) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
       }
       if (f < F) {
         float *ps = p.stats + ((size_t(kvh) * p.splits + split) * kMaxFused + f) * 2;
@@ -280,6 +309,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attention_tc_kernel(const AttnP
       const uint32_t b = i & 1, slot = i % kAtRaw;
       bool ok = at_wait(&raw_full[slot], (i / kAtRaw) & 1);
       if (ok && i >= 2) ok = at_wait(&kv_empty[b], ((i >> 1) - 1) & 1);
+      if (ok && i == 1) ok = at_wait(q_ready, 0);  // (Q is turned in the second buffers)
       if (!ok) {
         if (ctid == 0) atomicExch(p.status, SB_DEV_WAIT_EXPIRED);
         break;

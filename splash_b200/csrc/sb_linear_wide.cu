@@ -143,7 +143,17 @@ __device__ __forceinline__ bool wide_warp_wait(uint64_t *bar, uint32_t parity, b
 // One CTA per row slot (rows past `rows` are written as zeros): optional RMSNorm, the row's largest magnitude, a
 // power-of-two scale that keeps the values below 2^10, fp16, stored in the MMA's core-matrix order. Within every four
 // consecutive inputs the order is [0, 2, 1, 3]: the order in which the weight expansion produces its halves.
-constexpr int kWidePrepThreads = 256;
+// A chain of latencies (the row, its statistics, the row again), so a row has as many threads as fill whole rounds of its chunks,
+// every split's loads are in flight together and the norm's weights are fetched before the wait: 128 rows of 5120 take 5.3 us
+// (7.2 with 256 threads and loads one after the other), with seven splits to add 8.4 (13.2). Tried: eight rows by a cluster of
+// eight CTAs, so that stores are whole lines (10.9 and 25 us).
+constexpr uint32_t kWidePrepMost = 768;
+// Threads for rows of `chunks` chunks: as few rounds as kWidePrepMost allows, evenly filled.
+static uint32_t wide_prep_threads(uint32_t chunks) {
+  const uint32_t rounds = (chunks + kWidePrepMost - 1) / kWidePrepMost;
+  return (chunks + 32 * rounds - 1) / (32 * rounds) * 32;
+}
+constexpr int kWideSlotThreads = 256, kWideSlotRows = 8, kWideSlotWarps = kWideSlotThreads / 32;
 struct WidePrepParams {
   const uint16_t *x;
   const float *norm_w;
@@ -161,195 +171,214 @@ struct WidePrepParams {
   float *scales;
   uint16_t *normed_out;  // optional bf16 [rows][k]: the normalised rows (with norm_w), for the fp32 side projections of the same input
 };
-__global__ void __launch_bounds__(kWidePrepThreads) wide_prepare_kernel(const WidePrepParams p) {
-  __shared__ float red_s[2 * (kWidePrepThreads / 32)];
-  const uint32_t tok = blockIdx.x, tid = threadIdx.x;  // the row slot inside its block
+// Eight bf16 inputs as fp16 with the row's power of two taken out, in the [0, 2, 1, 3] order.
+__device__ __forceinline__ uint4 wide_pack(const float (&v)[8], float down) {
+  __half hv[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) hv[j] = __float2half_rn(v[j] * down);
+  const __half2 p0 = __halves2half2(hv[0], hv[2]), p1 = __halves2half2(hv[1], hv[3]);
+  const __half2 p2 = __halves2half2(hv[4], hv[6]), p3 = __halves2half2(hv[5], hv[7]);
+  return make_uint4(*reinterpret_cast<const uint32_t *>(&p0), *reinterpret_cast<const uint32_t *>(&p1), *reinterpret_cast<const uint32_t *>(&p2),
+                    *reinterpret_cast<const uint32_t *>(&p3));
+}
+__device__ __forceinline__ void wide_unpack(const uint4 raw, float (&v)[8]) {
+  const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[2 * j] = bf16_bits_to_float(u[j] & 0xffffu), v[2 * j + 1] = bf16_bits_to_float(u[j] >> 16);
+}
+// Where chunk c (8 inputs) of row slot `tok` stands in its block.
+__device__ __forceinline__ size_t wide_unit(uint32_t c, uint32_t tok, uint32_t rows_padded) {
+  const uint32_t k0 = 8 * c, unit = k0 / 64, step = (k0 % 64) / 16, half = (k0 % 16) / 8;
+  return size_t(unit) * rows_padded * 128 + size_t(step) * rows_padded * 32 + (tok >> 3) * 256 + half * 128 + (tok & 7) * 16;
+}
+// The power of two of a row whose largest magnitude is mx: scaled values stay below 2^10.
+__device__ __forceinline__ int wide_exponent(float mx) {
+  int e = 0;
+  if (mx > 0.0f && mx <= 3.0e38f) {
+    (void)frexpf(mx, &e);
+    e -= 10;
+  }
+  return e;
+}
+
+__global__ void __launch_bounds__(kWidePrepMost) wide_prepare_kernel(const WidePrepParams p) {
+  __shared__ float red_s[kWidePrepMost / 32][2];
+  const uint32_t tok = blockIdx.x, tid = threadIdx.x, threads = blockDim.x;  // the row slot inside its block
+  const uint32_t chunks = p.k / 8;                      // 8 inputs each
   pdl_launch_dependents();
+  // (the norm's weights do not depend on the kernel ahead)
+  if (p.norm_w && tok < p.rows)
+    for (uint32_t c = 4 * tid; c < chunks; c += 4 * threads) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.norm_w + 8 * c));
   pdl_wait();
   const bool live = tok < p.rows;
-  const uint32_t rows_padded = p.rows_padded;
   const uint16_t *xrow = p.x + size_t(tok) * p.x_stride;
-  uint8_t *block = p.out + kWideHeader;
-  float *scale_dst = reinterpret_cast<float *>(p.out) + tok;
-  const uint32_t chunks = p.k / 8;  // 8 inputs each
-  // A thread's chunks (tid, tid + 256, ...) stay in its registers from the pass that forms or first reads them to the
-  // conversion (up to kKeep of them: k <= 18432); a longer row is read again from memory, where this thread wrote it.
-  constexpr int kKeep = 9;
+  // A thread's chunks (tid, tid + threads, ...) stay in its registers from the pass that forms or first reads them to the
+  // conversion (up to kKeep of them); a longer row is read again from memory, where this thread wrote it.
+  constexpr int kKeep = 5;
   uint4 keep[kKeep];
-  const bool kept = chunks <= uint32_t(kKeep) * kWidePrepThreads;
-  if (p.partials && live) {
-    // The projection ahead left its k-splits' sums: add them in split order onto the residual, round once, and keep the
-    // rows (the new hidden state).
-    uint16_t *xw = const_cast<uint16_t *>(xrow);
-    auto sum_chunk = [&](uint32_t c) {
-      const uint4 raw = *reinterpret_cast<const uint4 *>(p.residual + size_t(tok) * p.residual_stride + 8 * c);
-      const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
-      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      for (uint32_t sp = 0; sp < p.splits; ++sp) {
-        const float4 *src = reinterpret_cast<const float4 *>(p.partials + (size_t(sp) * p.rows_total + p.row0 + tok) * p.partial_stride + 8 * c);
-        const float4 a = __ldcg(src), b = __ldcg(src + 1);
-        acc[0] += a.x, acc[1] += a.y, acc[2] += a.z, acc[3] += a.w, acc[4] += b.x, acc[5] += b.y, acc[6] += b.z, acc[7] += b.w;
-      }
-      uint32_t o[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t lo = float_to_bf16_bits(acc[2 * j] + bf16_bits_to_float(u[j] & 0xffffu));
-        const uint32_t hi = float_to_bf16_bits(acc[2 * j + 1] + bf16_bits_to_float(u[j] >> 16));
-        o[j] = lo | (hi << 16);
-      }
-      const uint4 out = make_uint4(o[0], o[1], o[2], o[3]);
-      *reinterpret_cast<uint4 *>(xw + 8 * c) = out;
-      return out;
-    };
-    if (kept) {
-#pragma unroll
-      for (int i = 0; i < kKeep; ++i) {
-        const uint32_t c = tid + uint32_t(i) * kWidePrepThreads;
-        if (c < chunks) keep[i] = sum_chunk(c);
-      }
-    } else {
-      for (uint32_t c = tid; c < chunks; c += kWidePrepThreads) (void)sum_chunk(c);
-    }
-  } else if (kept && live) {
-#pragma unroll
-    for (int i = 0; i < kKeep; ++i) {
-      const uint32_t c = tid + uint32_t(i) * kWidePrepThreads;
-      if (c < chunks) keep[i] = *reinterpret_cast<const uint4 *>(xrow + 8 * c);
-    }
-  }
+  const bool kept = chunks <= uint32_t(kKeep) * threads;
   float ss = 0.0f, mx = 0.0f;
   auto measure = [&](uint32_t c, const uint4 raw) {
-    const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+    float v[8];
+    wide_unpack(raw, v);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float a = bf16_bits_to_float(u[j] & 0xffffu), b = bf16_bits_to_float(u[j] >> 16);
-      ss = fmaf(a, a, ss), ss = fmaf(b, b, ss);
-      const float wa = p.norm_w ? p.norm_w[8 * c + 2 * j] : 1.0f, wb = p.norm_w ? p.norm_w[8 * c + 2 * j + 1] : 1.0f;
-      mx = fmaxf(mx, fmaxf(fabsf(a * wa), fabsf(b * wb)));
+    for (int j = 0; j < 8; ++j) ss = fmaf(v[j], v[j], ss);
+    if (p.norm_w) {
+      const float4 w0 = *reinterpret_cast<const float4 *>(p.norm_w + 8 * c), w1 = *reinterpret_cast<const float4 *>(p.norm_w + 8 * c + 4);
+      v[0] *= w0.x, v[1] *= w0.y, v[2] *= w0.z, v[3] *= w0.w, v[4] *= w1.x, v[5] *= w1.y, v[6] *= w1.z, v[7] *= w1.w;
     }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(v[j]));
   };
-  if (kept) {
+  // The projection ahead left its k-splits' sums: add them in split order onto the residual, round once, and keep the
+  // rows (the new hidden state).
+  auto sum_chunk = [&](uint32_t c) {
+    const uint4 raw = *reinterpret_cast<const uint4 *>(p.residual + size_t(tok) * p.residual_stride + 8 * c);
+    const float *src = p.partials + (size_t(p.row0) + tok) * p.partial_stride + 8 * c;
+    const size_t pitch = size_t(p.rows_total) * p.partial_stride;
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (uint32_t s0 = 0; s0 < p.splits; s0 += 4) {  // four splits' loads in flight
+      float4 a[4], b[4];
 #pragma unroll
-    for (int i = 0; i < kKeep; ++i) {
-      const uint32_t c = tid + uint32_t(i) * kWidePrepThreads;
-      if (c < chunks && live) measure(c, keep[i]);
+      for (int j = 0; j < 4; ++j) {
+        if (s0 + j >= p.splits) continue;
+        a[j] = __ldcg(reinterpret_cast<const float4 *>(src + (s0 + j) * pitch)), b[j] = __ldcg(reinterpret_cast<const float4 *>(src + (s0 + j) * pitch) + 1);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (s0 + j >= p.splits) continue;
+        acc[0] += a[j].x, acc[1] += a[j].y, acc[2] += a[j].z, acc[3] += a[j].w, acc[4] += b[j].x, acc[5] += b[j].y, acc[6] += b[j].z, acc[7] += b[j].w;
+      }
     }
-  } else {
-    for (uint32_t c = tid; c < chunks && live; c += kWidePrepThreads) measure(c, *reinterpret_cast<const uint4 *>(xrow + 8 * c));
+    float v[8];
+    wide_unpack(raw, v);
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      o[j] = uint32_t(float_to_bf16_bits(acc[2 * j] + v[2 * j])) | (uint32_t(float_to_bf16_bits(acc[2 * j + 1] + v[2 * j + 1])) << 16);
+    const uint4 out = make_uint4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<uint4 *>(const_cast<uint16_t *>(xrow) + 8 * c) = out;
+    return out;
+  };
+  if (live) {
+    if (kept) {
+      if (p.partials) {
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i)
+          if (tid + i * threads < chunks) keep[i] = sum_chunk(tid + i * threads);
+      } else {
+#pragma unroll
+        for (int i = 0; i < kKeep; ++i)
+          if (tid + i * threads < chunks) keep[i] = *reinterpret_cast<const uint4 *>(xrow + 8 * (tid + i * threads));
+      }
+#pragma unroll
+      for (int i = 0; i < kKeep; ++i)
+        if (tid + i * threads < chunks) measure(tid + i * threads, keep[i]);
+    } else {
+      for (uint32_t c = tid; c < chunks; c += threads) measure(c, p.partials ? sum_chunk(c) : *reinterpret_cast<const uint4 *>(xrow + 8 * c));
+    }
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     ss += __shfl_xor_sync(0xffffffffu, ss, o);
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   }
-  if ((tid & 31) == 0) red_s[2 * (tid >> 5)] = ss, red_s[2 * (tid >> 5) + 1] = mx;
+  if ((tid & 31) == 0) red_s[tid >> 5][0] = ss, red_s[tid >> 5][1] = mx;
   __syncthreads();
-  ss = red_s[0], mx = red_s[1];
-  for (int w = 1; w < kWidePrepThreads / 32; ++w) ss += red_s[2 * w], mx = fmaxf(mx, red_s[2 * w + 1]);
+  ss = red_s[0][0], mx = red_s[0][1];
+  for (uint32_t w = 1; w < threads / 32; ++w) ss += red_s[w][0], mx = fmaxf(mx, red_s[w][1]);
   float inv = 1.0f;
   if (p.norm_w) {
     inv = rsqrtf(ss / float(p.k) + 1e-6f);
     mx = mx * inv * 1.0625f;  // (x inv) w against x w inv and the rounding to bf16: well inside 6 %
   }
-  int e = 0;
-  if (mx > 0.0f && mx <= 3.0e38f) {
-    (void)frexpf(mx, &e);
-    e -= 10;
-  }
+  const int e = wide_exponent(mx);
   const float down = ldexpf(1.0f, -e);
-  if (tid == 0) *scale_dst = live ? ldexpf(1.0f, e) : 0.0f;
-  const size_t unit_bytes = size_t(rows_padded) * 128;  // 64 inputs of every row slot
+  if (tid == 0) reinterpret_cast<float *>(p.out)[tok] = live ? ldexpf(1.0f, e) : 0.0f;
   auto convert = [&](uint32_t c, const uint4 raw) {
-    uint32_t h[4] = {0, 0, 0, 0};
+    uint4 h = make_uint4(0, 0, 0, 0);
     if (live) {
-      const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
       float v[8];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) v[2 * j] = bf16_bits_to_float(u[j] & 0xffffu), v[2 * j + 1] = bf16_bits_to_float(u[j] >> 16);
+      wide_unpack(raw, v);
       if (p.norm_w) {
+        const float4 w0 = *reinterpret_cast<const float4 *>(p.norm_w + 8 * c), w1 = *reinterpret_cast<const float4 *>(p.norm_w + 8 * c + 4);
+        const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = round_bf16((v[j] * inv) * p.norm_w[8 * c + j]);
+        for (int j = 0; j < 8; ++j) v[j] = round_bf16((v[j] * inv) * w[j]);
         if (p.normed_out) {
           uint32_t n[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) n[j] = float_to_bf16_bits(v[2 * j]) | (float_to_bf16_bits(v[2 * j + 1]) << 16);
+          for (int j = 0; j < 4; ++j) n[j] = uint32_t(float_to_bf16_bits(v[2 * j])) | (uint32_t(float_to_bf16_bits(v[2 * j + 1])) << 16);
           *reinterpret_cast<uint4 *>(p.normed_out + size_t(tok) * p.k + 8 * c) = make_uint4(n[0], n[1], n[2], n[3]);
         }
       }
-      __half hv[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) hv[j] = __float2half_rn(v[j] * down);
-      const __half2 p0 = __halves2half2(hv[0], hv[2]), p1 = __halves2half2(hv[1], hv[3]);
-      const __half2 p2 = __halves2half2(hv[4], hv[6]), p3 = __halves2half2(hv[5], hv[7]);
-      h[0] = *reinterpret_cast<const uint32_t *>(&p0), h[1] = *reinterpret_cast<const uint32_t *>(&p1);
-      h[2] = *reinterpret_cast<const uint32_t *>(&p2), h[3] = *reinterpret_cast<const uint32_t *>(&p3);
+      h = wide_pack(v, down);
     }
-    const uint32_t k0 = 8 * c, unit = k0 / 64, step = (k0 % 64) / 16, half = (k0 % 16) / 8;
-    uint8_t *dst = block + unit * unit_bytes + size_t(step) * rows_padded * 32 + (tok >> 3) * 256 + half * 128 + (tok & 7) * 16;
-    *reinterpret_cast<uint4 *>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4 *>(p.out + kWideHeader + wide_unit(c, tok, p.rows_padded)) = h;
   };
   if (kept) {
 #pragma unroll
-    for (int i = 0; i < kKeep; ++i) {
-      const uint32_t c = tid + uint32_t(i) * kWidePrepThreads;
-      if (c < chunks) convert(c, live ? keep[i] : make_uint4(0, 0, 0, 0));
-    }
+    for (int i = 0; i < kKeep; ++i)
+      if (tid + i * threads < chunks) convert(tid + i * threads, keep[i]);
   } else {
-    for (uint32_t c = tid; c < chunks; c += kWidePrepThreads) convert(c, live ? *reinterpret_cast<const uint4 *>(xrow + 8 * c) : make_uint4(0, 0, 0, 0));
+    for (uint32_t c = tid; c < chunks; c += threads) convert(c, live ? *reinterpret_cast<const uint4 *>(xrow + 8 * c) : make_uint4(0, 0, 0, 0));
   }
 }
 
-// The conversion of the groups' row slots with a warp per slot (no norm, no sums to add): a slot's table look-ups and its row
-// are a short chain, so many slots a CTA and few CTAs beat a CTA per slot (an MoE block's 6700 slots were 27 us as a CTA each).
-constexpr int kWideSlotWarps = 8;
-__global__ void __launch_bounds__(32 * kWideSlotWarps) wide_prepare_slots_kernel(const WidePrepParams p) {
+// The conversion of the groups' row slots (no norm, no sums to add): a CTA eight neighbouring slots, which are eight rows of one
+// group's block (groups begin at multiples of 16 slots), lanes as above. (An MoE block of 512 rows, both conversions of its 6700
+// slots: 318 us instead of 324 with a warp a slot, whose stores were 16 bytes of a line; a CTA a slot was slower still.)
+__global__ void __launch_bounds__(kWideSlotThreads) wide_prepare_slots_kernel(const WidePrepParams p) {
+  __shared__ float warp_s[kWideSlotWarps][kWideSlotRows];
   pdl_launch_dependents();
   pdl_wait();
-  const uint32_t slot = blockIdx.x * kWideSlotWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (slot >= __ldg(p.slot_count)) return;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, slot = blockIdx.x * kWideSlotRows + (tid & 7);
+  if (blockIdx.x * kWideSlotRows >= __ldg(p.slot_count)) return;
   const uint32_t src = __ldg(p.slot_src + slot), sg = __ldg(p.slot_group + slot);
   const uint4 rec = __ldg(p.groups + (sg >> 8));
   const bool live = src != 0xffffffffu;
   const uint32_t tok = sg & 0xffu, rows_padded = rec.w, chunks = p.k / 8;
   const uint16_t *xrow = p.x + size_t(live ? src : 0) * p.x_stride;
   uint8_t *block = p.out + size_t(rec.y) * p.k * 2;
+  constexpr uint32_t kStep = kWideSlotThreads / kWideSlotRows;
+  constexpr int kKeep = 8;  // chunks a thread keeps (k <= 2048); the others are read again
+  uint4 keep[kKeep];
   float mx = 0.0f;
-  for (uint32_t c = lane; c < chunks && live; c += 32) {
-    const uint4 raw = *reinterpret_cast<const uint4 *>(xrow + 8 * c);
-    const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+  auto measure = [&](const uint4 raw) {
+    float v[8];
+    wide_unpack(raw, v);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) mx = fmaxf(mx, fmaxf(fabsf(bf16_bits_to_float(u[j] & 0xffffu)), fabsf(bf16_bits_to_float(u[j] >> 16))));
-  }
+    for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(v[j]));
+  };
 #pragma unroll
-  for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  int e = 0;
-  if (mx > 0.0f && mx <= 3.0e38f) {
-    (void)frexpf(mx, &e);
-    e -= 10;
-  }
+  for (int i = 0; i < kKeep; ++i)
+    if (live && (tid >> 3) + i * kStep < chunks) keep[i] = *reinterpret_cast<const uint4 *>(xrow + 8 * ((tid >> 3) + i * kStep));
+#pragma unroll
+  for (int i = 0; i < kKeep; ++i)
+    if (live && (tid >> 3) + i * kStep < chunks) measure(keep[i]);
+  for (uint32_t c = (tid >> 3) + kKeep * kStep; live && c < chunks; c += kStep) measure(*reinterpret_cast<const uint4 *>(xrow + 8 * c));
+#pragma unroll
+  for (int o = 16; o >= 8; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane < kWideSlotRows) warp_s[warp][lane] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kWideSlotWarps; ++w) mx = fmaxf(mx, warp_s[w][tid & 7]);
+  const int e = wide_exponent(mx);
   const float down = ldexpf(1.0f, -e);
-  if (lane == 0) p.scales[slot] = live ? ldexpf(1.0f, e) : 0.0f;
-  const size_t unit_bytes = size_t(rows_padded) * 128;
-  for (uint32_t c = lane; c < chunks; c += 32) {
-    uint32_t h[4] = {0, 0, 0, 0};
+  if (tid < kWideSlotRows) p.scales[slot] = live ? ldexpf(1.0f, e) : 0.0f;
+  auto convert = [&](uint32_t c, const uint4 raw) {
+    uint4 h = make_uint4(0, 0, 0, 0);
     if (live) {
-      const uint4 raw = *reinterpret_cast<const uint4 *>(xrow + 8 * c);
-      const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
-      __half hv[8];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        hv[2 * j] = __float2half_rn(bf16_bits_to_float(u[j] & 0xffffu) * down);
-        hv[2 * j + 1] = __float2half_rn(bf16_bits_to_float(u[j] >> 16) * down);
-      }
-      const __half2 p0 = __halves2half2(hv[0], hv[2]), p1 = __halves2half2(hv[1], hv[3]);
-      const __half2 p2 = __halves2half2(hv[4], hv[6]), p3 = __halves2half2(hv[5], hv[7]);
-      h[0] = *reinterpret_cast<const uint32_t *>(&p0), h[1] = *reinterpret_cast<const uint32_t *>(&p1);
-      h[2] = *reinterpret_cast<const uint32_t *>(&p2), h[3] = *reinterpret_cast<const uint32_t *>(&p3);
+      float v[8];
+      wide_unpack(raw, v);
+      h = wide_pack(v, down);
     }
-    const uint32_t k0 = 8 * c, unit = k0 / 64, step = (k0 % 64) / 16, half = (k0 % 16) / 8;
-    uint8_t *dst = block + unit * unit_bytes + size_t(step) * rows_padded * 32 + (tok >> 3) * 256 + half * 128 + (tok & 7) * 16;
-    *reinterpret_cast<uint4 *>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
-  }
+    *reinterpret_cast<uint4 *>(block + wide_unit(c, tok, rows_padded)) = h;
+  };
+#pragma unroll
+  for (int i = 0; i < kKeep; ++i)
+    if ((tid >> 3) + i * kStep < chunks) convert((tid >> 3) + i * kStep, keep[i]);
+  for (uint32_t c = (tid >> 3) + kKeep * kStep; c < chunks; c += kStep) convert(c, live ? *reinterpret_cast<const uint4 *>(xrow + 8 * c) : make_uint4(0, 0, 0, 0));
 }
 
 // The four sub-blocks 4h .. 4h+3 of a Q4_K row's super-block as 128 halves in 64 packed columns:
@@ -836,7 +865,7 @@ int launch_wide_prepare_grouped(cudaStream_t stream, const WidePrepareGroupedArg
   pp.x = static_cast<const uint16_t *>(a.x), pp.out = static_cast<uint8_t *>(a.prepared), pp.k = a.k, pp.x_stride = a.x_stride;
   pp.slot_src = a.slot_src, pp.slot_group = a.slot_group, pp.slot_count = a.slot_count, pp.groups = a.groups, pp.scales = a.scales;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((a.max_slots + kWideSlotWarps - 1) / kWideSlotWarps), cfg.blockDim = dim3(32 * kWideSlotWarps), cfg.stream = stream;
+  cfg.gridDim = dim3((a.max_slots + kWideSlotRows - 1) / kWideSlotRows), cfg.blockDim = dim3(kWideSlotThreads), cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -1074,7 +1103,7 @@ static int wide_prepare(void *stream, const void *x, uint32_t rows, uint32_t k, 
                       splits, rows, r0, partial_stride, residual_stride};
     pp.normed_out = normed_out ? static_cast<uint16_t *>(normed_out) + size_t(r0) * k : nullptr;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(padded), cfg.blockDim = dim3(kWidePrepThreads), cfg.stream = as_stream(stream);
+    cfg.gridDim = dim3(padded), cfg.blockDim = dim3(wide_prep_threads(k / 8)), cfg.stream = as_stream(stream);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;

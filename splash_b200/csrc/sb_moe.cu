@@ -336,25 +336,33 @@ __global__ void __launch_bounds__(kMoeGroupThreads) moe_group_kernel(const uint3
                                                                      uint32_t *status, MoeShare share) {
   __shared__ uint16_t warp_count[kMoeGroupWarps][kMoeMaxExperts];  // then: the place of the warp's next route of the expert
   __shared__ uint32_t count_s[kMoeMaxExperts], slot0_s[kMoeMaxExperts], group0_s[kMoeMaxExperts];
+  extern __shared__ uint16_t place_s[];  // [n] the routes' experts' places, kNoPlace for those the launch does not take
+  constexpr uint32_t kNoPlace = 0xffffu;
   pdl_launch_dependents();
-  pdl_wait();
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (uint32_t i = tid; i < kMoeGroupWarps * kMoeMaxExperts; i += kMoeGroupThreads) (&warp_count[0][0])[i] = 0;
-  __syncthreads();
+  pdl_wait();
   const uint32_t run = ((n + kMoeGroupWarps - 1) / kMoeGroupWarps + 31) / 32 * 32, first = warp * run, last = min(n, first + run);
   const uint32_t lt = (1u << lane) - 1u;
-  auto expert_at = [&](uint32_t i) -> uint32_t {
-    if (i >= last) return 0xffffffffu;
+  // Every route's expert once, all threads' loads in flight together.
+#pragma unroll 4
+  for (uint32_t i = tid; i < n; i += kMoeGroupThreads) {
     const uint32_t e = selected[i];
+    uint32_t place = kNoPlace;
     if (e == share.shared_id) {
       const uint32_t row = i / routes;
-      return row >= share.own_row0 && row - share.own_row0 < share.own_rows ? share.local : 0xffffffffu;
-    }
-    if (e - share.expert0 < share.local) return e - share.expert0;
-    if (share.expert0 == 0 && share.shared_id == 0xffffffffu && share.local == experts) {  // a whole block: an id outside it breaks the contract
-      atomicCAS(status, 0u, uint32_t(SB_DEV_CONTRACT));
-    }
-    return 0xffffffffu;  // another rank's expert (or a dropped route)
+      if (row >= share.own_row0 && row - share.own_row0 < share.own_rows) place = share.local;
+    } else if (e - share.expert0 < share.local) {
+      place = e - share.expert0;
+    } else if (share.expert0 == 0 && share.shared_id == 0xffffffffu && share.local == experts) {
+      atomicCAS(status, 0u, uint32_t(SB_DEV_CONTRACT));  // a whole block: an id outside it breaks the contract
+    }  // (else another rank's expert, or a dropped route)
+    place_s[i] = uint16_t(place);
+  }
+  __syncthreads();
+  auto expert_at = [&](uint32_t i) -> uint32_t {
+    const uint32_t e = i < last ? place_s[i] : kNoPlace;
+    return e == kNoPlace ? 0xffffffffu : e;
   };
   for (uint32_t i0 = first; i0 < last; i0 += 32) {
     const uint32_t e = expert_at(i0 + lane);
@@ -386,24 +394,25 @@ __global__ void __launch_bounds__(kMoeGroupThreads) moe_group_kernel(const uint3
         if (lane >= uint32_t(o)) gs += a, ss += b;
       }
       const uint32_t my_group = group + gs - groups, my_slot = slot + ss - slots;
-      if (e < experts) {
-        slot0_s[e] = my_slot, group0_s[e] = my_group;
-        for (uint32_t k = 0; k < groups; ++k) {
-          const uint32_t rows = min(c - k * kMoeGroupRows, kMoeGroupRows);
-          g.groups[my_group + k] = make_uint4(e, my_slot + k * kMoeGroupRows, rows, (rows + 15) / 16 * 16);
-        }
-        // the padding slots behind the expert's last route
-        const uint32_t lastg = my_group + (groups ? groups - 1 : 0);
-        for (uint32_t r = c; r < slots; ++r) {
-          g.slot_src[my_slot + r] = 0xffffffffu, g.slot_self[my_slot + r] = 0xffffffffu;
-          g.slot_group[my_slot + r] = (lastg << 8) | (r - (lastg - my_group) * kMoeGroupRows);
-        }
-      }
+      if (e < experts) slot0_s[e] = my_slot, group0_s[e] = my_group;
       group += __shfl_sync(0xffffffffu, gs, 31), slot += __shfl_sync(0xffffffffu, ss, 31);
     }
     if (lane == 0) g.counts[0] = group, g.counts[1] = slot;
   }
   __syncthreads();
+  // A thread per expert: its groups, and the padding slots behind its last route.
+  for (uint32_t e = tid; e < experts; e += kMoeGroupThreads) {
+    const uint32_t c = count_s[e], groups = (c + kMoeGroupRows - 1) / kMoeGroupRows, slots = (c + 15) / 16 * 16, my_slot = slot0_s[e], my_group = group0_s[e];
+    for (uint32_t k = 0; k < groups; ++k) {
+      const uint32_t rows = min(c - k * kMoeGroupRows, kMoeGroupRows);
+      g.groups[my_group + k] = make_uint4(e, my_slot + k * kMoeGroupRows, rows, (rows + 15) / 16 * 16);
+    }
+    const uint32_t lastg = my_group + (groups ? groups - 1 : 0);
+    for (uint32_t r = c; r < slots; ++r) {
+      g.slot_src[my_slot + r] = 0xffffffffu, g.slot_self[my_slot + r] = 0xffffffffu;
+      g.slot_group[my_slot + r] = (lastg << 8) | (r - (lastg - my_group) * kMoeGroupRows);
+    }
+  }
   for (uint32_t i0 = first; i0 < last; i0 += 32) {
     const uint32_t i = i0 + lane, e = expert_at(i);
     const uint32_t same = __match_any_sync(0xffffffffu, e);
@@ -423,30 +432,63 @@ __global__ void __launch_bounds__(kMoeGroupThreads) moe_group_kernel(const uint3
 
 // out = bf16(residual + sum over the row's routes in slot order of weight * float(y)), y at the routes' row slots.
 // partial != 0: the routes the launch took only (slot_of_route says which: the others hold ~0), fp32 sums without the residual.
+// A thread eight columns, eight routes' values in flight.
 __global__ void __launch_bounds__(256) moe_combine_grouped_kernel(const SbMoeExpertArgs a, const uint32_t *slot_of_route, const uint16_t *y, uint32_t partial) {
+  __shared__ uint32_t slot_s[32];
+  __shared__ float weight_s[32];
   pdl_launch_dependents();
   pdl_wait();
-  const uint32_t row = blockIdx.y, c = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
+  const uint32_t row = blockIdx.y, c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (threadIdx.x < a.routes) slot_s[threadIdx.x] = slot_of_route[row * a.routes + threadIdx.x], weight_s[threadIdx.x] = a.weights[row * a.routes + threadIdx.x];
+  __syncthreads();
   if (c >= a.hidden) return;
-  float acc0 = 0.0f, acc1 = 0.0f;
-  for (uint32_t s = 0; s < a.routes; ++s) {
-    const uint32_t route = row * a.routes + s, slot = slot_of_route[route];
-    if (slot == 0xffffffffu) continue;  // (not taken by the grouping)
-    const float w = a.weights[route];
-    const uint32_t pair = *reinterpret_cast<const uint32_t *>(y + size_t(slot) * a.hidden + c);
-    acc0 += w * bf16_bits_to_float(pair & 0xffffu), acc1 += w * bf16_bits_to_float(pair >> 16);
+  float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+  for (uint32_t s0 = 0; s0 < a.routes; s0 += 8) {
+    uint4 v[8];
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j)
+      if (s0 + j < a.routes && slot_s[s0 + j] != 0xffffffffu) v[j] = *reinterpret_cast<const uint4 *>(y + size_t(slot_s[s0 + j]) * a.hidden + c);
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) {
+      if (s0 + j >= a.routes || slot_s[s0 + j] == 0xffffffffu) continue;  // (not taken by the grouping)
+      const float w = weight_s[s0 + j];
+      const uint32_t u[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[2 * i] += w * bf16_bits_to_float(u[i] & 0xffffu), acc[2 * i + 1] += w * bf16_bits_to_float(u[i] >> 16);
+    }
   }
   if (partial) {
-    *reinterpret_cast<float2 *>(static_cast<float *>(a.out) + size_t(row) * a.hidden + c) = make_float2(acc0, acc1);
+    float *out = static_cast<float *>(a.out) + size_t(row) * a.hidden + c;
+    if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+      *reinterpret_cast<float4 *>(out) = make_float4(acc[0], acc[1], acc[2], acc[3]), *reinterpret_cast<float4 *>(out + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) *reinterpret_cast<float2 *>(out + i) = make_float2(acc[i], acc[i + 1]);
+    }
     return;
   }
-  float r0 = 0.0f, r1 = 0.0f;
-  if (a.residual) {
-    const uint32_t pair = *reinterpret_cast<const uint32_t *>(static_cast<const uint16_t *>(a.residual) + size_t(row) * a.hidden + c);
-    r0 = bf16_bits_to_float(pair & 0xffffu), r1 = bf16_bits_to_float(pair >> 16);
+  // (rows that lie on four bytes only are read and written two values at a time)
+  const uint16_t *residual = a.residual ? static_cast<const uint16_t *>(a.residual) + size_t(row) * a.hidden + c : nullptr;
+  uint16_t *out = static_cast<uint16_t *>(a.out) + size_t(row) * a.hidden + c;
+  uint32_t r[4] = {0, 0, 0, 0};
+  if (residual) {
+    if ((reinterpret_cast<uintptr_t>(residual) & 15) == 0) {
+      const uint4 w = *reinterpret_cast<const uint4 *>(residual);
+      r[0] = w.x, r[1] = w.y, r[2] = w.z, r[3] = w.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = reinterpret_cast<const uint32_t *>(residual)[i];
+    }
   }
-  *reinterpret_cast<uint32_t *>(static_cast<uint16_t *>(a.out) + size_t(row) * a.hidden + c) =
-      uint32_t(float_to_bf16_bits(r0 + acc0)) | (uint32_t(float_to_bf16_bits(r1 + acc1)) << 16);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    r[i] = uint32_t(float_to_bf16_bits(bf16_bits_to_float(r[i] & 0xffffu) + acc[2 * i])) | (uint32_t(float_to_bf16_bits(bf16_bits_to_float(r[i] >> 16) + acc[2 * i + 1])) << 16);
+  if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    *reinterpret_cast<uint4 *>(out) = make_uint4(r[0], r[1], r[2], r[3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) reinterpret_cast<uint32_t *>(out)[i] = r[i];
+  }
 }
 
 template <class K> static int launch_moe(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const MoeParams &p) {
@@ -483,7 +525,10 @@ static int moe_experts_grouped(cudaStream_t s, const SbMoeExpertArgs *a, const M
   const bool pdl = ctx().pdl;
   {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1), cfg.blockDim = dim3(kMoeGroupThreads), cfg.stream = s;
+    static std::atomic<uint64_t> allowed;
+    const int st = allow_smem(reinterpret_cast<const void *>(moe_group_kernel), kMoeMaxRoutes * sizeof(uint16_t), allowed);
+    if (st != SB_OK) return st;
+    cfg.gridDim = dim3(1), cfg.blockDim = dim3(kMoeGroupThreads), cfg.dynamicSmemBytes = n * sizeof(uint16_t), cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -508,7 +553,7 @@ static int moe_experts_grouped(cudaStream_t s, const SbMoeExpertArgs *a, const M
   st = launch_linear_wide_grouped(s, down);
   if (st != SB_OK) return st;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((a->hidden / 2 + 255) / 256, a->rows), cfg.blockDim = dim3(256), cfg.stream = s;
+  cfg.gridDim = dim3((a->hidden / 8 + 255) / 256, a->rows), cfg.blockDim = dim3(std::min(256u, a->hidden / 8)), cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;

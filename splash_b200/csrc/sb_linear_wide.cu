@@ -138,6 +138,9 @@ __device__ __forceinline__ bool wide_warp_wait(uint64_t *bar, uint32_t parity, b
   if ((threadIdx.x & 31) == 0) ok = backoff ? mbar_wait_backoff(bar, parity) : mbar_wait(bar, parity);
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
+// The same for the hand-over that paces the kernel: every lane polls and none parks. The vote gives all lanes one outcome and
+// brings the warp together for the tensor-memory stores that follow, which take whole warps.
+__device__ __forceinline__ bool wide_warp_spin(uint64_t *bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_spin(bar, parity)); }
 
 // ---- the conversion of X ----
 // One CTA per row slot (rows past `rows` are written as zeros): optional RMSNorm, the row's largest magnitude, a
@@ -684,7 +687,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) linear_wide_kernel(const Wide
           // itself (a MoE block of 512 rows 320.6 -> 306 us, a feed-forward block of 128 rows 104.0 -> 102.2). Finer
           // hand-overs, so that a buffer's first half is refilled while its second is read, cost more than they hide: 128 rows
           // gate / up 49.0 -> 56.3 us.
-          if (scount > 0 && !mbar_wait_spin(&a_empty[ab], (scount - 1) & 1)) {
+          if (scount > 0 && !wide_warp_spin(&a_empty[ab], (scount - 1) & 1)) {
             if (lane == 0) wide_expired(p.status, 7);
             ok = false;
             break;

@@ -201,11 +201,11 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
   // Only a caller that vouches for the cell (SB_GDN_STATE_SETTLED: nothing still running on the stream writes
   // state_in) gets the early load; otherwise the launch ahead may be the one that produced the cell (a fold
   // followed at once by a step on the swapped cells), and the load waits for it like every other read.
-  const float a_scale = a.a_scale[h], dt_bias = bf16_bits_to_float(static_cast<const uint16_t *>(a.dt_bias)[h]);  // (weights)
   const bool settled = (a.flags & SB_GDN_STATE_SETTLED) != 0;
   if (settled) load_state();
   pdl_wait();
   if (!settled) load_state();
+  const float a_scale = a.a_scale[h], dt_bias = bf16_bits_to_float(static_cast<const uint16_t *>(a.dt_bias)[h]);
   // Conv inputs of this CTA's channels (q and k of the key head, 32 value dimensions), in[3 + row][local channel], and their taps'
   // weights: asynchronous copies, on their way while the gate projection runs.
   const uint32_t chan0[3] = {kh * kD, KW + kh * kD, 2 * KW + h * kD + vd0};

@@ -147,7 +147,7 @@ __device__ __forceinline__ bool wide_warp_spin(uint64_t *bar, uint32_t parity) {
 // power-of-two scale that keeps the values below 2^10, fp16, stored in the MMA's core-matrix order. Within every four
 // consecutive inputs the order is [0, 2, 1, 3]: the order in which the weight expansion produces its halves.
 // A chain of latencies (the row, its statistics, the row again), so a row has as many threads as fill whole rounds of its chunks,
-// every split's loads are in flight together and the norm's weights are fetched before the wait: 128 rows of 5120 take 5.3 us
+// every split's loads are in flight together and the norm's weights are fetched beside the row: 128 rows of 5120 take 5.3 us
 // (7.2 with 256 threads and loads one after the other), with seven splits to add 8.4 (13.2). Tried: eight rows by a cluster of
 // eight CTAs, so that stores are whole lines (10.9 and 25 us).
 constexpr uint32_t kWidePrepMost = 768;
@@ -209,10 +209,10 @@ __global__ void __launch_bounds__(kWidePrepMost) wide_prepare_kernel(const WideP
   const uint32_t tok = blockIdx.x, tid = threadIdx.x, threads = blockDim.x;  // the row slot inside its block
   const uint32_t chunks = p.k / 8;                      // 8 inputs each
   pdl_launch_dependents();
-  // (the norm's weights do not depend on the kernel ahead)
+  pdl_wait();
+  // The norm's weights on their way beside the row. (Behind the wait like every other read: the kernel ahead may have written them.)
   if (p.norm_w && tok < p.rows)
     for (uint32_t c = 4 * tid; c < chunks; c += 4 * threads) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.norm_w + 8 * c));
-  pdl_wait();
   const bool live = tok < p.rows;
   const uint16_t *xrow = p.x + size_t(tok) * p.x_stride;
   // A thread's chunks (tid, tid + threads, ...) stay in its registers from the pass that forms or first reads them to the

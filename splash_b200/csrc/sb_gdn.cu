@@ -34,6 +34,7 @@
 //            (pending_rows, or a device word written by sb_accept) to the next step, which folds them
 #include <algorithm>
 #include <cooperative_groups.h>
+#include <type_traits>
 
 #include "sb_internal.h"
 #include "sb_ptx.cuh"
@@ -420,20 +421,24 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
   // The unknowns of state row `lane`, by one warp: u_t = beta_t (v_t - m_t), m_t = D_t (S k_t) (in sh.u) + sum over j < t of c[j][t] u_j,
   // a finished unknown at a time so that a step waits for three operations only. What the state already holds of v_t is summed by
   // itself: it is small beside v_t, so its roundings are too (with -beta c u_j added to the right-hand side one by one the folded
-  // state was 8e-8 off instead of 6e-8).
-  auto solve = [&](const float (*c)[kGramPitch], const float (&v)[kGdnRows][kGdnVd], const float (&beta)[kGdnRows], float (&u)[kGdnRows]) {
+  // state was 8e-8 off instead of 6e-8). A tree row takes the unknowns on its own path only (not the others times zero: one of them
+  // may be no number); in a chain every earlier unknown is on it.
+  auto solve = [&](auto tree_rows, const float (*c)[kGramPitch], const float (&v)[kGdnRows][kGdnVd], const float (&beta)[kGdnRows], float (&u)[kGdnRows]) {
+    constexpr bool kPaths = decltype(tree_rows)::value;
+    const uint32_t path = kPaths ? sh.path[lane % kGdnRows] : 0u;
 #pragma unroll
     for (int t = 0; t < kGdnRows; ++t) u[t] = sh.u[t][lane];
 #pragma unroll
     for (int j = 0; j < kGdnRows; ++j) {
       u[j] = beta[j] * (v[j][lane] - u[j]);
+      const uint32_t takes = kPaths ? __ballot_sync(0xffffffffu, path >> j & 1u) : 0xffffffffu;  // the rows with j on their path
 #pragma unroll
       for (int t4x = (j + 1) / 4 * 4; t4x < kGdnRows; t4x += 4) {
         const float4 c4 = *reinterpret_cast<const float4 *>(&c[j][t4x]);
-        if (t4x > j) u[t4x] = fmaf(c4.x, u[j], u[t4x]);
-        if (t4x + 1 > j) u[t4x + 1] = fmaf(c4.y, u[j], u[t4x + 1]);
-        if (t4x + 2 > j) u[t4x + 2] = fmaf(c4.z, u[j], u[t4x + 2]);
-        if (t4x + 3 > j) u[t4x + 3] = fmaf(c4.w, u[j], u[t4x + 3]);
+        if (t4x > j && (takes >> t4x & 1u)) u[t4x] = fmaf(c4.x, u[j], u[t4x]);
+        if (t4x + 1 > j && (takes >> (t4x + 1) & 1u)) u[t4x + 1] = fmaf(c4.y, u[j], u[t4x + 1]);
+        if (t4x + 2 > j && (takes >> (t4x + 2) & 1u)) u[t4x + 2] = fmaf(c4.z, u[j], u[t4x + 2]);
+        if (t4x + 3 > j && (takes >> (t4x + 3) & 1u)) u[t4x + 3] = fmaf(c4.w, u[j], u[t4x + 3]);
       }
     }
   };
@@ -485,12 +490,13 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
     __syncthreads();
     if (warp == 0) {
       float u[kGdnRows];
-      solve(sh.kk, sh.pv, sh.pbeta, u);
+      solve(std::false_type{}, sh.kk, sh.pv, sh.pbeta, u);
 #pragma unroll
       for (int t4x = 0; t4x < kGdnRows; t4x += 4) {
         const float4 g4x = *reinterpret_cast<const float4 *>(&sh.after[t4x]);
-        sh.u[t4x][lane] = g4x.x * u[t4x], sh.u[t4x + 1][lane] = g4x.y * u[t4x + 1];
-        sh.u[t4x + 2][lane] = g4x.z * u[t4x + 2], sh.u[t4x + 3][lane] = g4x.w * u[t4x + 3];
+        const float g[4] = {g4x.x, g4x.y, g4x.z, g4x.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sh.u[t4x + i][lane] = uint32_t(t4x + i) < pending ? g[i] * u[t4x + i] : 0.0f;
       }
     }
   }
@@ -613,19 +619,22 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
   __syncthreads();
   if (warp == 0) {
     float u[kGdnRows];
-    solve(sh.pkk, sh.v, sh.beta, u);
+    solve(std::bool_constant<kTree>{}, sh.pkk, sh.v, sh.beta, u);
 #pragma unroll
     for (int t = 0; t < kGdnRows; ++t) sh.u[t][lane] = u[t];
   }
   __syncthreads();
   for (uint32_t t = warp; t < rows; t += kGdnThreads / 32) {
+    const uint32_t path = sh.path[t];
     float o = sh.o[t][lane];
 #pragma unroll
-    for (int j4 = 0; j4 < kGdnRows; j4 += 4) {  // (coefficients past t are zeros)
+    for (int j4 = 0; j4 < kGdnRows; j4 += 4) {  // the rows on its path (the others may hold no numbers)
       if (uint32_t(j4) > t) break;
       const float4 c4 = *reinterpret_cast<const float4 *>(&sh.kq[t][j4]);
-      o = fmaf(c4.x, sh.u[j4][lane], o), o = fmaf(c4.y, sh.u[j4 + 1][lane], o);
-      o = fmaf(c4.z, sh.u[j4 + 2][lane], o), o = fmaf(c4.w, sh.u[j4 + 3][lane], o);
+      if (path >> j4 & 1u) o = fmaf(c4.x, sh.u[j4][lane], o);
+      if (path >> (j4 + 1) & 1u) o = fmaf(c4.y, sh.u[j4 + 1][lane], o);
+      if (path >> (j4 + 2) & 1u) o = fmaf(c4.z, sh.u[j4 + 2][lane], o);
+      if (path >> (j4 + 3) & 1u) o = fmaf(c4.w, sh.u[j4 + 3][lane], o);
     }
     head_ctas.map_shared_rank(&sh.out[t % 4][vd0 + lane], int(t / 4))[0] = round_bf16(o);
   }

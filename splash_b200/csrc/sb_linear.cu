@@ -480,11 +480,7 @@ template <bool TP> __global__ void __launch_bounds__(kPrepThreads) prepare_kerne
       }
     }
   }
-  int e = 0;
-  if (mx > 0.0f && mx <= 3.0e38f) {
-    (void)frexpf(mx, &e);  // mx = f * 2^e with f in [0.5, 1): scaled values stay below 2^10
-    e -= 10;
-  }
+  const int e = row_exponent(mx);
   const float down = ldexpf(1.0f, -e);
   if (tid == 0 && rank == 0) reinterpret_cast<float *>(p.out)[tok] = ldexpf(1.0f, e);
   const uint32_t h = tok >> 3, g = tok & 7;

@@ -194,15 +194,6 @@ __device__ __forceinline__ size_t wide_unit(uint32_t c, uint32_t tok, uint32_t r
   const uint32_t k0 = 8 * c, unit = k0 / 64, step = (k0 % 64) / 16, half = (k0 % 16) / 8;
   return size_t(unit) * rows_padded * 128 + size_t(step) * rows_padded * 32 + (tok >> 3) * 256 + half * 128 + (tok & 7) * 16;
 }
-// The power of two of a row whose largest magnitude is mx: scaled values stay below 2^10.
-__device__ __forceinline__ int wide_exponent(float mx) {
-  int e = 0;
-  if (mx > 0.0f && mx <= 3.0e38f) {
-    (void)frexpf(mx, &e);
-    e -= 10;
-  }
-  return e;
-}
 
 __global__ void __launch_bounds__(kWidePrepMost) wide_prepare_kernel(const WidePrepParams p) {
   __shared__ float red_s[kWidePrepMost / 32][2];
@@ -295,7 +286,7 @@ __global__ void __launch_bounds__(kWidePrepMost) wide_prepare_kernel(const WideP
     inv = rsqrtf(ss / float(p.k) + 1e-6f);
     mx = mx * inv * 1.0625f;  // (x inv) w against x w inv and the rounding to bf16: well inside 6 %
   }
-  const int e = wide_exponent(mx);
+  const int e = row_exponent(mx);
   const float down = ldexpf(1.0f, -e);
   if (tid == 0) reinterpret_cast<float *>(p.out)[tok] = live ? ldexpf(1.0f, e) : 0.0f;
   auto convert = [&](uint32_t c, const uint4 raw) {
@@ -366,7 +357,7 @@ __global__ void __launch_bounds__(kWideSlotThreads) wide_prepare_slots_kernel(co
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < kWideSlotWarps; ++w) mx = fmaxf(mx, warp_s[w][tid & 7]);
-  const int e = wide_exponent(mx);
+  const int e = row_exponent(mx);
   const float down = ldexpf(1.0f, -e);
   if (tid < kWideSlotRows) p.scales[slot] = live ? ldexpf(1.0f, e) : 0.0f;
   auto convert = [&](uint32_t c, const uint4 raw) {

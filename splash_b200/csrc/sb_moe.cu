@@ -58,7 +58,8 @@ struct MoeParams {
   float *x_scale, *act_scale;
 };
 
-// A bf16 row in fp16 with a power of two taken out (exact for values down to 2^-24 of the row's largest), in the order a lane of
+// A bf16 row in fp16 with a power of two taken out (exact for values down to 2^-26 of the row's largest, smaller ones to within 2^-34
+// of it), in the order a lane of
 // the expert kernels reads it: unit (i2, p, t) of a super-block holds inputs 32 (2 t + p) + 8 i2 .. + 7 as [0,2,1,3,4,6,5,7] (the
 // order the Q4_K nibbles come out in), and lane t's 8 bytes of sums are sub-blocks 2 t, 2 t + 1, each a high and a low half.
 __device__ __forceinline__ void moe_convert_row(const uint16_t *src, uint32_t k, uint8_t *dst, float *scale, float *scratch) {
@@ -89,11 +90,7 @@ __device__ __forceinline__ void moe_convert_row(const uint16_t *src, uint32_t k,
   if ((tid & 31) == 0) scratch[tid >> 5] = mx;
   __syncthreads();
   for (uint32_t w = 0; w < blockDim.x / 32; ++w) mx = fmaxf(mx, scratch[w]);
-  int e = 0;
-  if (mx > 0.0f && mx <= 3.0e38f) {
-    (void)frexpf(mx, &e);
-    e -= 10;  // scaled values stay below 2^10
-  }
+  const int e = row_exponent(mx);
   const float down = ldexpf(1.0f, -e);
   if (tid == 0) *scale = ldexpf(1.0f, e);
 #pragma unroll

@@ -175,6 +175,18 @@ __device__ __forceinline__ uint16_t float_to_bf16_bits(float f) {
 }
 __device__ __forceinline__ float round_bf16(float f) { return __bfloat162float(__float2bfloat16_rn(f)); }
 
+// The exponent of the power of two taken out of a row of fp16 inputs whose largest magnitude is mx (0: none): scaled values stay below
+// 2^10. Never below -126, so that 2^-e stays finite for rows near bf16's smallest magnitudes (their scaled values are then
+// smaller, and still exact: bf16 reaches down to 2^-133). A row with an infinity keeps its values.
+__device__ __forceinline__ int row_exponent(float mx) {
+  int e = 0;
+  if (mx > 0.0f && mx < INFINITY) {
+    (void)frexpf(mx, &e);  // mx = f * 2^e with f in [0.5, 1)
+    e = max(e - 10, -126);
+  }
+  return e;
+}
+
 // e^-x as exp2(-x log2 e): the form every activation of the verify step uses.
 // The quotient is the approximate one (reciprocal and multiply, 2 ulp): every result is rounded to bf16 next.
 __device__ __forceinline__ float silu_f(float x) { return __fdividef(x, 1.0f + exp2f(-1.44269504089f * x)); }

@@ -173,7 +173,7 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
   const uint32_t KH = a.key_heads, VH = a.value_heads, KW = KH * kD, VW = VH * kD, C = 2 * KW + VW;
   const uint32_t per_key = VH / KH, kh = h / per_key, vd0 = vs * kGdnVd;
   const uint32_t rows = a.rows;
-  const bool fused_gates = a.gate_weight && rows > 0;
+  const bool projects = a.gate_weight && 4 * vs < rows;  // this CTA has rows of the fused gate projection
   const uint16_t *qkvz = static_cast<const uint16_t *>(a.qkvz);
   const uint16_t *conv_w = static_cast<const uint16_t *>(a.conv_w);
   const uint16_t *cs_in = static_cast<const uint16_t *>(a.conv_state_in);
@@ -234,7 +234,7 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
   // {b, a} over the layer's normalised input and stores them into all four CTAs of the head; the rows' threads add the
   // 8 groups in order below (the order of sb_linear_f32, so the bits agree with the unfused way).
   float gates[4][2];
-  if (fused_gates) {
+  if (projects) {
     const float *const wrow[2] = {a.gate_weight + size_t(h) * a.gate_k, a.gate_weight + size_t(VH + h) * a.gate_k};
     const uint16_t *gx = static_cast<const uint16_t *>(a.gate_input);
     const uint16_t *xrow[4];
@@ -254,7 +254,7 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
     copy_async<16>(&sh.in[r][lc], hsrc >= 0 ? pin + size_t(pending_row(uint32_t(hsrc))) * C + ch : cs_in + size_t(3 + hsrc) * C + ch);
   }
   // pending rows' keys, values and gates from their tape, requested before the gate projection's lanes are added up and stored
-  // after; rows past them are zeros (the products below take whole eights)
+  // after; rows past them are zeros to a whole eight (the products below take eights)
   constexpr int kPkLoads = kGdnRows * kD / 2 / kGdnThreads, kPvLoads = kGdnRows * kGdnVd / kGdnThreads;
   uint32_t pk2[kPkLoads];
   uint16_t pv1[kPvLoads], pbeta1 = 0;
@@ -276,7 +276,7 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
   // The gates' eight sums over the lanes, halved at every exchange: lane l ends with sum l / 4 (row l / 8, b or a). The same
   // additions as a butterfly of each, so the same bits.
   float gate_sum = 0.0f;
-  if (fused_gates) {
+  if (projects) {
     float v[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = gates[i >> 1][i & 1];
@@ -296,6 +296,7 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
 #pragma unroll
   for (int i = 0; i < kPkLoads; ++i) {
     const uint32_t n = tid / (kD / 2) + i * (kGdnThreads / (kD / 2));
+    if (n >= (pending + 7) / 8 * 8) break;
     *reinterpret_cast<float2 *>(&sh.pk[n][2 * (tid % (kD / 2))]) = make_float2(bf16_bits_to_float(pk2[i] & 0xffffu), bf16_bits_to_float(pk2[i] >> 16));
   }
 #pragma unroll
@@ -323,7 +324,7 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
   };
   __syncthreads();  // the CTA's staging is complete
   cluster_wait();   // every CTA of the head runs
-  if (fused_gates) head_ctas.map_shared_rank(&sh.gate[warp][4 * vs + (lane >> 3)][(lane >> 2) & 1], int(lane & 3))[0] = gate_sum;
+  if (projects) head_ctas.map_shared_rank(&sh.gate[warp][4 * vs + (lane >> 3)][(lane >> 2) & 1], int(lane & 3))[0] = gate_sum;
   if (warp >= 4 && 4 * (warp - 4) + vs < pending) inner_products(pending_key, pending_key(4 * (warp - 4) + vs), sh.pkk, 4 * (warp - 4) + vs);
   cluster_arrive();  // (1) the gates' sums and the pending rows' inner products
   // NC neighbouring channels' convolution and SiLU for a row.
@@ -372,8 +373,8 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
 #pragma unroll
     for (int peer = 0; peer < kGdnSplit; ++peer) *reinterpret_cast<uint2 *>(head_ctas.map_shared_rank(vec, peer)) = make_uint2(bits[0], bits[1]);
   }
-  // (rows past the block are zeros: the products take all sixteen)
-  for (uint32_t i = tid; i < (kGdnRows - rows) * (kD / 2); i += kGdnThreads)
+  // (rows past the block are zeros to a whole eight: the products take eights, the inner products' of further rows are not used)
+  for (uint32_t i = tid; i < ((rows + 7) / 8 * 8 - rows) * (kD / 2); i += kGdnThreads)
     *reinterpret_cast<uint32_t *>(&sh.x[0][rows + i / (kD / 2)][2 * (i % (kD / 2))]) = *reinterpret_cast<uint32_t *>(&sh.x[1][rows + i / (kD / 2)][2 * (i % (kD / 2))]) = 0u;
   // Two values of a row a thread, here and below: row ct, value dimensions 2 cj, + 1.
   const uint32_t ct = tid / kGdnRows, cj = tid % kGdnRows, cv = 2 * cj;
@@ -418,18 +419,19 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
     }
     return g;
   };
-  // The unknowns of state row `lane`, by one warp: u_t = beta_t (v_t - m_t), m_t = D_t (S k_t) (in sh.u) + sum over j < t of c[j][t] u_j,
+  // The n unknowns of state row `lane`, by one warp: u_t = beta_t (v_t - m_t), m_t = D_t (S k_t) (in sh.u) + sum over j < t of c[j][t] u_j,
   // a finished unknown at a time so that a step waits for three operations only. What the state already holds of v_t is summed by
   // itself: it is small beside v_t, so its roundings are too (with -beta c u_j added to the right-hand side one by one the folded
   // state was 8e-8 off instead of 6e-8). A tree row takes the unknowns on its own path only (not the others times zero: one of them
   // may be no number); in a chain every earlier unknown is on it.
-  auto solve = [&](auto tree_rows, const float (*c)[kGramPitch], const float (&v)[kGdnRows][kGdnVd], const float (&beta)[kGdnRows], float (&u)[kGdnRows]) {
+  auto solve = [&](auto tree_rows, uint32_t n, const float (*c)[kGramPitch], const float (&v)[kGdnRows][kGdnVd], const float (&beta)[kGdnRows], float (&u)[kGdnRows]) {
     constexpr bool kPaths = decltype(tree_rows)::value;
     const uint32_t path = kPaths ? sh.path[lane % kGdnRows] : 0u;
 #pragma unroll
     for (int t = 0; t < kGdnRows; ++t) u[t] = sh.u[t][lane];
 #pragma unroll
     for (int j = 0; j < kGdnRows; ++j) {
+      if (uint32_t(j) >= n) break;
       u[j] = beta[j] * (v[j][lane] - u[j]);
       const uint32_t takes = kPaths ? __ballot_sync(0xffffffffu, path >> j & 1u) : 0xffffffffu;  // the rows with j on their path
 #pragma unroll
@@ -444,12 +446,13 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
   };
   if (pending) {  // (3)
     __syncthreads();  // nobody reads the convolution inputs any more (they have been read since the CTA arrived)
-    // S pk_t: eight rows at a time, a thread its two state rows over its eight columns, summed over the four lanes that share
-    // the rows (products halved at every exchange).
-    for (uint32_t n0 = 0; n0 < pending; n0 += 8) {
-      float v[16];  // [row of the pair][pending row]
+    // S pk_t: eight rows at a time (four where there are no more), a thread its two state rows over its eight columns, summed over
+    // the four lanes that share the rows (products halved at every exchange).
+    auto products = [&](auto count, uint32_t n0) {
+      constexpr int N = decltype(count)::value;
+      float v[2 * N];  // [row of the pair][pending row]
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
+      for (int n = 0; n < N; ++n) {
         float lo = 0.0f, hi = 0.0f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {  // block c / 2, pair c % 2
@@ -458,20 +461,25 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
           lo = fmaf(S[at], k2.x, lo), lo = fmaf(S[at + 1], k2.y, lo);
           hi = fmaf(S[at + 4], k2.x, hi), hi = fmaf(S[at + 5], k2.y, hi);
         }
-        v[n] = lo, v[8 + n] = hi;
+        v[n] = lo, v[N + n] = hi;
       }
 #pragma unroll
-      for (int half = 8; half >= 4; half >>= 1) {  // lanes 2 apart divide the pair's rows, lanes 1 apart the eight products
-        const bool upper = (lane & (half >> 2)) != 0;
+      for (int half = N; half >= N / 2; half >>= 1) {  // lanes 2 apart divide the pair's rows, lanes 1 apart the products
+        const int apart = half == N ? 2 : 1;
+        const bool upper = (lane & apart) != 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < N; ++i) {
           if (i >= half) break;
           const float give = upper ? v[i] : v[i + half], keep = upper ? v[i + half] : v[i];
-          v[i] = keep + __shfl_xor_sync(0xffffffffu, give, half >> 2);
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, give, apart);
         }
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) sh.part[quarter][n0 + 4 * (lane & 1) + i][srow + ((lane & 2) ? 8 : 0)] = v[i];
+      for (int i = 0; i < N / 2; ++i) sh.part[quarter][n0 + N / 2 * (lane & 1) + i][srow + ((lane & 2) ? 8 : 0)] = v[i];
+    };
+    for (uint32_t n0 = 0; n0 < pending; n0 += 8) {
+      if (pending - n0 > 4) products(std::integral_constant<int, 8>{}, n0);
+      else products(std::integral_constant<int, 4>{}, n0);
     }
     __syncthreads();
     // coefficients [j][t] (into the matrix the block's rows use later) and D_t (S k_t); rows past the pending ones are zeros
@@ -485,18 +493,19 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
       right = make_float2(d * sx.x, d * sx.y);
     }
     *reinterpret_cast<float2 *>(&sh.u[ct][cv]) = right;
-    if (cj == 0) sh.after[ct] = decays(sh.pdecay, ((1u << pending) - 1u) & ~((2u << ct) - 1u));
+    if (there && cj == 0) sh.after[ct] = decays(sh.pdecay, ((1u << pending) - 1u) & ~((2u << ct) - 1u));
     if (tid == 1) sh.pending_decay = decays(sh.pdecay, (1u << pending) - 1u);
     __syncthreads();
     if (warp == 0) {
       float u[kGdnRows];
-      solve(std::false_type{}, sh.kk, sh.pv, sh.pbeta, u);
+      solve(std::false_type{}, pending, sh.kk, sh.pv, sh.pbeta, u);
 #pragma unroll
       for (int t4x = 0; t4x < kGdnRows; t4x += 4) {
         const float4 g4x = *reinterpret_cast<const float4 *>(&sh.after[t4x]);
         const float g[4] = {g4x.x, g4x.y, g4x.z, g4x.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sh.u[t4x + i][lane] = uint32_t(t4x + i) < pending ? g[i] * u[t4x + i] : 0.0f;
+        for (int i = 0; i < 4; ++i)
+          if (uint32_t(t4x + i) < pending) sh.u[t4x + i][lane] = g[i] * u[t4x + i];
       }
     }
   }
@@ -529,9 +538,10 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
     const float d = sh.pending_decay;
 #pragma unroll
     for (int i = 0; i < 16; ++i) S[i] *= d;
-    for (uint32_t t0 = 0; t0 < pending; t0 += 2) {  // (rows past the pending ones are zeros)
+    for (uint32_t t0 = 0; t0 < pending; t0 += 2) {
 #pragma unroll
       for (uint32_t t = t0; t < t0 + 2; ++t) {
+        if (t >= pending) break;
         const float u0 = sh.u[t][srow], u1 = sh.u[t][srow + 8];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -572,6 +582,7 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
       }
 #pragma unroll
       for (int n = 0; n < 4; ++n) {  // k rows 0-7, 8-15, q rows 0-7, 8-15
+        if ((n & 1) && rows <= 8) continue;
         const uint16_t *x = &sh.x[n >> 1][8 * (n & 1) + g4][scol + 16 * b];
         const uint32_t b0 = *reinterpret_cast<const uint32_t *>(x), b1 = *reinterpret_cast<const uint32_t *>(x + 8);
         mma_bf16(acc[n], lo[0], lo[1], lo[2], lo[3], b0, b1);
@@ -582,7 +593,8 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) sh.part[quarter][8 * n + 2 * t4 + (i & 1)][srow + 8 * (i >> 1)] = acc[n][i];
+      for (int i = 0; i < 4; ++i)
+        if (!(n & 1) || rows > 8) sh.part[quarter][8 * n + 2 * t4 + (i & 1)][srow + 8 * (i >> 1)] = acc[n][i];
   }
   if (qk_writer)
     for (uint32_t i = tid; i < rows * kD / 2; i += kGdnThreads)
@@ -619,7 +631,7 @@ __global__ void __cluster_dims__(kGdnSplit, 1, 1) __launch_bounds__(kGdnThreads,
   __syncthreads();
   if (warp == 0) {
     float u[kGdnRows];
-    solve(std::bool_constant<kTree>{}, sh.pkk, sh.v, sh.beta, u);
+    solve(std::bool_constant<kTree>{}, rows, sh.pkk, sh.v, sh.beta, u);
 #pragma unroll
     for (int t = 0; t < kGdnRows; ++t) sh.u[t][lane] = u[t];
   }

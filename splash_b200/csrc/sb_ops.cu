@@ -526,12 +526,21 @@ __device__ __forceinline__ void sample_row(const SbSampleArgs &a, uint32_t r) {
   a.selected[r] = pick;
 }
 
-// grid (8 rows, lanes), a cluster a row; `cluster` false: grid (rows, lanes), a block a row.
-template <bool CLUSTER> __global__ void __launch_bounds__(CLUSTER ? kSelectThreads : kSampleThreads, CLUSTER ? 2 : 1) sample_kernel(const SbSampleArgs a) {
+// Whether a greedy lane's rows take a CTA each, eight neighbouring rows a cluster and the lane's other clusters none, in a launch whose
+// lanes have policies of their own (known on the device only): where it has more rows than a greedy launch gives a cluster each.
+constexpr uint32_t kGreedyClusterRows = 32;
+__device__ __forceinline__ bool alone_in_cluster(const SbSampleArgs &a, uint32_t lane) {
+  return a.rows * max(a.lanes, 1u) > kGreedyClusterRows && a.lane_policies[lane].temperature == 0.0f;
+}
+
+// grid (8 rows, lanes), a cluster a row (POLICIES: or a CTA); `cluster` false: grid (rows, lanes), a block a row.
+template <bool CLUSTER, bool POLICIES = false> __global__ void __launch_bounds__(CLUSTER ? kSelectThreads : kSampleThreads, CLUSTER ? 2 : 1) sample_kernel(const SbSampleArgs a) {
   extern __shared__ __align__(16) uint8_t select_smem[];
   pdl_launch_dependents();
   pdl_wait();
-  if (CLUSTER) {
+  if (POLICIES && alone_in_cluster(a, blockIdx.y)) {
+    if (blockIdx.x < a.rows) greedy_row(lane_selection(a, blockIdx.y), blockIdx.x);
+  } else if (CLUSTER) {
     SelectRow::sync();  // every CTA of the row runs before any writes into it
     select_row(lane_selection(a, blockIdx.y), blockIdx.x / kSelectCtas, select_smem);
   } else {
@@ -600,24 +609,29 @@ __device__ __forceinline__ void commit_lane(const SbSelectAcceptArgs &c, uint32_
 // Selection, acceptance and the lane's commit in one launch: a cluster (or block) per row selects, and the one of a
 // lane that finishes last (a ticket per lane, drawn after the row's selection is visible) walks the accepted path
 // and commits the lane. The ticket word returns to zero for the next launch.
-template <bool CLUSTER> __global__ void __launch_bounds__(CLUSTER ? kSelectThreads : kSampleThreads, CLUSTER ? 2 : 1) select_accept_kernel(const SbSelectAcceptArgs c_in) {
+template <bool CLUSTER, bool POLICIES = false> __global__ void __launch_bounds__(CLUSTER ? kSelectThreads : kSampleThreads, CLUSTER ? 2 : 1) select_accept_kernel(const SbSelectAcceptArgs c_in) {
   extern __shared__ __align__(16) uint8_t select_smem[];
   pdl_launch_dependents();
   pdl_wait();
-  const uint32_t lane = blockIdx.y, row = CLUSTER ? blockIdx.x / kSelectCtas : blockIdx.x;
+  const uint32_t lane = blockIdx.y;
+  const bool alone = POLICIES && alone_in_cluster(c_in.sample, lane);
+  const uint32_t row = CLUSTER && !alone ? blockIdx.x / kSelectCtas : blockIdx.x;
+  if (POLICIES && row >= c_in.sample.rows) return;
   // The lane's own rows (blocks of different lengths step together): the blocks of the slots past them select nothing.
   const uint32_t lane_rows = c_in.lane_rows ? min(c_in.lane_rows[lane], c_in.sample.rows) : c_in.sample.rows;
   if (row < lane_rows) {
     SbSampleArgs s = lane_selection(c_in.sample, lane);
     s.rows = lane_rows;
-    if (CLUSTER) {
+    if (alone) {
+      greedy_row(s, row);
+    } else if (CLUSTER) {
       SelectRow::sync();  // every CTA of the row runs before any writes into it
       select_row(s, row, select_smem);
     } else {
       sample_row(s, row);
     }
   }
-  if (CLUSTER && blockIdx.x % kSelectCtas) return;
+  if (CLUSTER && !alone && blockIdx.x % kSelectCtas) return;
   if (threadIdx.x != 0) return;
   __threadfence();
   if (atomicAdd(c_in.tickets + lane, 1u) != c_in.sample.rows - 1) return;
@@ -756,9 +770,9 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const SbMoeRouteArgs a) 
 // for one CTA a SM only (above some 160,000 ids): without filters 128 rows of 232,001 take 220 us against 259, 512 rows 804
 // against 800, so from 256 such rows on a row is a block's; with filters clusters win at every count (512 rows: 2.1 ms
 // against 34.6).
-constexpr uint32_t kGreedyClusterRows = 32, kPlainClusterRows = 256;
+constexpr uint32_t kPlainClusterRows = 256;
 constexpr size_t kTwoCtasSmem = 113 * 1024;
-template <class A> static int launch_selection(void (*cluster)(A), void (*block)(A), const SbSampleArgs &s, cudaStream_t stream, const A &args) {
+template <class A> static int launch_selection(void (*cluster)(A), void (*policies)(A), void (*block)(A), const SbSampleArgs &s, cudaStream_t stream, const A &args) {
   const bool staged = s.lane_policies || (s.temperature != 0.0f && s.uniforms);
   const uint32_t rows = s.rows * std::max(1u, s.lanes);
   const bool filtered = s.lane_policies || s.min_p > 0.0f || (s.top_k > 0 && s.top_k < s.vocab) || (s.top_p > 0.0f && s.top_p < 1.0f);
@@ -777,8 +791,9 @@ template <class A> static int launch_selection(void (*cluster)(A), void (*block)
   cfg.attrs = attr;
   cfg.numAttrs = clusters ? 2 : 1;
   if (clusters) {
-    static std::atomic<uint64_t> allowed;  // (one a kind of arguments, that is, one a kernel)
-    const int st = allow_smem(reinterpret_cast<const void *>(cluster), select_smem_bytes(kSelectVocab), allowed);
+    static std::atomic<uint64_t> allowed[2];  // (a pair a kind of arguments, that is, one a kernel)
+    if (s.lane_policies) cluster = policies;
+    const int st = allow_smem(reinterpret_cast<const void *>(cluster), select_smem_bytes(kSelectVocab), allowed[s.lane_policies ? 1 : 0]);
     if (st != SB_OK) return st;
   }
   SB_CUDA(cudaLaunchKernelEx(&cfg, clusters ? cluster : block, args));
@@ -921,7 +936,7 @@ int sb_sample_verify(void *stream, const SbSampleArgs *a) {
   SB_REQUIRE(!a->candidate_ids || (a->candidate_q && a->draws), "sb_sample_verify: candidates come with their draft probabilities and the rows' draws");
   SB_REQUIRE(a->lanes <= 64, "sb_sample_verify: %u lanes (up to 64)", a->lanes);
   SB_REQUIRE(!a->lane_policies || (a->uniforms && a->workspace && a->vocab <= kSelectVocab), "sb_sample_verify: policies a lane need uniforms, the workspace and a vocabulary the filters take");
-  return launch_selection(sample_kernel<true>, sample_kernel<false>, *a, as_stream(stream), *a);
+  return launch_selection(sample_kernel<true>, sample_kernel<true, true>, sample_kernel<false>, *a, as_stream(stream), *a);
 }
 
 int sb_sample_admit(void *stream, const SbAdmitArgs *a) {
@@ -973,7 +988,7 @@ int sb_select_accept(void *stream, const SbSelectAcceptArgs *c) {
   SB_REQUIRE(b->n_stop == 0 || b->stop_tokens, "sb_select_accept: stop tokens missing");
   SB_REQUIRE(!c->committed || (c->pending_rows && c->pending_path), "sb_select_accept: the commit needs the lanes' pending words");
   SB_REQUIRE((c->advance & 0xffu) <= 3 && ((c->advance & 0xffu) != 3 || c->advance >> 8 == a->rows), "sb_select_accept: advance = 0x%x", c->advance);
-  return launch_selection(select_accept_kernel<true>, select_accept_kernel<false>, *a, as_stream(stream), *c);
+  return launch_selection(select_accept_kernel<true>, select_accept_kernel<true, true>, select_accept_kernel<false>, *a, as_stream(stream), *c);
 }
 
 int sb_accept(void *stream, const SbAcceptArgs *a) {

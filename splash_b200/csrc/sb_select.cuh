@@ -546,6 +546,70 @@ struct SelectRow {
   }
 };
 
+// Tokens v0 .. v0 + n - 1 from src on, by a CTA of kSelectThreads: the best of them and how many can be selected, a warp's in all
+// its lanes; keep(logit, place) sees every one of them.
+template <int FLIGHT, class K> __device__ __forceinline__ void best_of(const float *src, uint32_t v0, uint32_t n, float &bv, uint32_t &bi, uint32_t &n_sel, K keep) {
+  const uint32_t tid = threadIdx.x;
+  bv = -INFINITY, bi = kSentinel, n_sel = 0;
+  auto take = [&](float x, uint32_t i) {
+    keep(x, i);
+    if (!selectable(x)) return;
+    ++n_sel;
+    if (bi == kSentinel || x > bv) bv = x, bi = v0 + i;  // (ids come in rising order)
+  };
+  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {  // rows that start on 16 bytes: FLIGHT 16-byte loads in flight
+    const uint32_t n4 = n / 4;
+    for (uint32_t i0 = tid; i0 < n4; i0 += FLIGHT * kSelectThreads) {
+      float4 x[FLIGHT];
+#pragma unroll
+      for (int j = 0; j < FLIGHT; ++j) {
+        const uint32_t i = i0 + j * kSelectThreads;
+        if (i < n4) x[j] = reinterpret_cast<const float4 *>(src)[i];
+      }
+#pragma unroll
+      for (int j = 0; j < FLIGHT; ++j) {
+        const uint32_t i = i0 + j * kSelectThreads;
+        if (i < n4) take(x[j].x, 4 * i), take(x[j].y, 4 * i + 1), take(x[j].z, 4 * i + 2), take(x[j].w, 4 * i + 3);
+      }
+    }
+    if (tid < (n & 3u)) take(src[4 * n4 + tid], 4 * n4 + tid);
+  } else {
+    for (uint32_t i0 = tid; i0 < n; i0 += 8 * kSelectThreads) {
+      float x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t i = i0 + j * kSelectThreads;
+        if (i < n) x[j] = src[i];
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (i0 + j * kSelectThreads < n) take(x[j], i0 + j * kSelectThreads);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+    const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (!better_token(bv, bi, ov, oi)) bv = ov, bi = oi;
+    n_sel += __shfl_xor_sync(0xffffffffu, n_sel, o);
+  }
+}
+
+// A greedy row's selection by one CTA of the cluster (the others have rows of their own).
+__device__ __forceinline__ void greedy_row(const SbSampleArgs &a, uint32_t r) {
+  __shared__ float best_v[kSelectWarps];
+  __shared__ uint32_t best_i[kSelectWarps];
+  float bv;
+  uint32_t bi, n_sel;
+  best_of<8>(a.logits + size_t(r) * a.logit_stride, 0, a.vocab, bv, bi, n_sel, [](float, uint32_t) {});
+  if ((threadIdx.x & 31) == 0) best_v[threadIdx.x >> 5] = bv, best_i[threadIdx.x >> 5] = bi;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < kSelectWarps; ++w)
+    if (!better_token(bv, bi, best_v[w], best_i[w])) bv = best_v[w], bi = best_i[w];
+  a.selected[r] = bi;
+}
+
 // One row's selection by the eight CTAs of a cluster; a is the row's lane's view. Thread 0 of CTA 0 writes it.
 __device__ __forceinline__ void select_row(const SbSampleArgs &a, uint32_t r, uint8_t *smem) {
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x % kSelectCtas;
@@ -560,51 +624,11 @@ __device__ __forceinline__ void select_row(const SbSampleArgs &a, uint32_t r, ui
   const bool sampled = a.temperature != 0.0f && a.uniforms;
   if (sampled && tid < 8 && row.shards + tid < padded) row.mass_ge[row.shards + tid] = row.mass_gt[row.shards + tid] = 0.0f;
   // The row's eighth: greedy choice and, for a sampled row, its copy in shared memory.
-  float bv = -INFINITY;
-  uint32_t bi = kSentinel, n_sel = 0;
-  const float *src = row.l + row.v0;
-  auto take = [&](float x, uint32_t i) {
+  float bv;
+  uint32_t bi, n_sel;
+  best_of<4>(row.l + row.v0, row.v0, row.n_mine, bv, bi, n_sel, [&](float x, uint32_t i) {
     if (sampled) row.slice[SelectRow::slot(i)] = token_key(x);
-    if (!selectable(x)) return;
-    ++n_sel;
-    if (bi == kSentinel || x > bv) bv = x, bi = row.v0 + i;  // (ids come in rising order)
-  };
-  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {  // rows that start on 16 bytes: four 16-byte loads in flight
-    const uint32_t n4 = row.n_mine / 4;
-    for (uint32_t i0 = tid; i0 < n4; i0 += 4 * kSelectThreads) {
-      float4 x[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t i = i0 + j * kSelectThreads;
-        if (i < n4) x[j] = reinterpret_cast<const float4 *>(src)[i];
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t i = i0 + j * kSelectThreads;
-        if (i < n4) take(x[j].x, 4 * i), take(x[j].y, 4 * i + 1), take(x[j].z, 4 * i + 2), take(x[j].w, 4 * i + 3);
-      }
-    }
-    if (tid < (row.n_mine & 3u)) take(src[4 * n4 + tid], 4 * n4 + tid);
-  } else {
-    for (uint32_t i0 = tid; i0 < row.n_mine; i0 += 8 * kSelectThreads) {
-      float x[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t i = i0 + j * kSelectThreads;
-        if (i < row.n_mine) x[j] = src[i];
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (i0 + j * kSelectThreads < row.n_mine) take(x[j], i0 + j * kSelectThreads);
-    }
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-    const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (!better_token(bv, bi, ov, oi)) bv = ov, bi = oi;
-    n_sel += __shfl_xor_sync(0xffffffffu, n_sel, o);
-  }
+  });
   if (lane == 0) sh.best_v[warp] = bv, sh.best_i[warp] = bi, sh.warp_count[0][warp] = n_sel;
   __syncthreads();
   if (tid < kSelectCtas) {

@@ -154,3 +154,43 @@ def test_the_two_kernels_select_alike(temperature, vocab, sides):
     assert np.array_equal(got[0][:common], got[1][:common])
     if temperature == 0.0:
         assert np.array_equal(got[1], np.concatenate([np.roll(base, 977 * z, axis=1).argmax(axis=1) for z in range(lanes)]))
+
+
+@pytest.mark.parametrize("lanes,rows,vocab", [(1, 16, 3000), (2, 16, 50257), (3, 13, 3001), (9, 16, 200000), (64, 5, 2049)])
+def test_policies_a_lane_equal_launches_of_one_policy(lanes, rows, vocab):
+    """Greedy lanes among sampled ones (their rows take a CTA each where the launch has many): the tokens of a launch with the lane's
+    policy for all."""
+    from splash_b200 import lib
+    lib.init(0)
+    l = lib.ops()
+    rng = np.random.default_rng(lanes * 100 + rows)
+    base = (rng.standard_normal((16, vocab)) * 2).astype(np.float32)
+    base[1, 7:19] = 30.0
+    base[2] = np.nan
+    logits = lib.DeviceBuffer(lanes * base.nbytes + 16)
+    for z in range(lanes):
+        logits.upload(np.roll(base, 977 * z, axis=1), offset=z * base.nbytes)
+    policies = [(0.0, 0.0, 0, 1.0), (0.7, 0.0, 50, 0.95), (0.9, 0.02, 0, 1.0)]
+    idd = lib.DeviceBuffer.from_numpy(rng.integers(0, vocab, (lanes, 16)).astype(np.uint32))
+    ud = lib.DeviceBuffer.from_numpy(rng.random((lanes, 80)).astype(np.float32))
+    wd = lib.DeviceBuffer(int(l.sb_sample_workspace_bytes(lanes * 16, vocab)))
+
+    def select(policy, table=None):
+        sd = lib.DeviceBuffer(lanes * 16 * 4)
+        sd.fill(0)
+        a = lib.SbSampleArgs(logits.ptr, idd.ptr, ud.ptr, sd.ptr, wd.ptr, rows, vocab, vocab, *policy)
+        a.lanes = lanes if lanes > 1 else 0
+        if table is not None:
+            a.lane_policies = table.ptr
+        lib.check(l.sb_sample_verify(None, ctypes.byref(a)))
+        lib.stream_sync()
+        assert lib.device_status() == 0
+        return sd.to_numpy(np.uint32, (lanes, 16))[:, :rows]
+
+    one = [select(p) for p in policies]
+    for shift, kinds in ((0, 3), (1, 3), (0, 1)):
+        which = [(z + shift) % kinds for z in range(lanes)]
+        table = lib.DeviceBuffer.from_numpy(np.frombuffer(bytes((lib.SbLanePolicy * lanes)(*[lib.SbLanePolicy(*policies[k]) for k in which])), np.uint8).copy())
+        got = select(policies[1], table)
+        for z in range(lanes):
+            assert np.array_equal(got[z], one[which[z]][z]), (z, which[z])

@@ -271,6 +271,120 @@ template <bool PAIR> __global__ void __launch_bounds__(kMoeThreads, 2) moe_few_k
   }
 }
 
+// ---- a few routes of small experts: a matrix-vector product a route ----
+// A warp computes eight output columns of a route against the staged row, a lane eight consecutive weights of every super-block: all
+// loads of a product in flight, three launches a block. It costs three instructions a weight and route, so it is the better one
+// only where the routes are few and the experts small (kMoeVectorWeights below).
+constexpr int kMoeColsPair = 8, kMoeColsDown = 8;  // output columns a warp computes (gate/up pass, down pass)
+constexpr float kMoeVectorDown = 0x1p-8f;          // on the inputs, taken back by the scales: eight products with codes up to 15 stay finite
+
+// scale and min of sub-block j of a Q4_K super-block from its 12 packed bytes (three words), in registers: bytes 0-3
+// hold the low 6 bits of scales 0-3 (and in their top 2 bits the high bits of scales 4-7), bytes 4-7 the same for the mins,
+// bytes 8-11 the low nibbles of scales 4-7 (low half) and mins 4-7 (high half).
+__device__ __forceinline__ void q4k_scale_min(const uint32_t (&w)[3], uint32_t j, float &sc, float &mn) {
+  const uint32_t s8 = 8 * (j & 3);
+  uint32_t isc, imn;
+  if (j < 4) {
+    isc = (w[0] >> s8) & 63u, imn = (w[1] >> s8) & 63u;
+  } else {
+    isc = ((w[2] >> s8) & 0xFu) | (((w[0] >> (s8 + 6)) & 3u) << 4);
+    imn = ((w[2] >> (s8 + 4)) & 0xFu) | (((w[1] >> (s8 + 6)) & 3u) << 4);
+  }
+  sc = float(isc), mn = float(imn);
+}
+
+// acc[m][c] += lane's share of dot(row c of matrix m, x) for NC consecutive Q4_K rows of each of NM matrices; x staged in
+// shared memory as floats; lane l takes weights 32 (l / 4) + 8 (l % 4) .. + 7 of every super-block, so the lane's x values
+// and their sum are fetched once per super-block for all the rows.
+template <int NM, int NC>
+__device__ __forceinline__ void q4k_rows_dot(const uint8_t *const (&rows)[NM], size_t row_bytes, const float *x, uint32_t k, uint32_t lane,
+                                             float (&acc)[NM][NC]) {
+  const uint32_t sub = lane >> 2, t0 = 8 * (lane & 3), shift = (sub & 1) * 4;
+#pragma unroll
+  for (int m = 0; m < NM; ++m)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[m][c] = 0.0f;
+#pragma unroll 2
+  for (uint32_t sb = 0; sb < k / 256; ++sb) {
+    const float4 x0 = *reinterpret_cast<const float4 *>(x + 256 * sb + 32 * sub + t0), x1 = *reinterpret_cast<const float4 *>(x + 256 * sb + 32 * sub + t0 + 4);
+    const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    const float xsum = ((xs[0] + xs[1]) + (xs[2] + xs[3])) + ((xs[4] + xs[5]) + (xs[6] + xs[7]));
+#pragma unroll
+    for (int m = 0; m < NM; ++m)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const uint8_t *blk = rows[m] + size_t(c) * row_bytes + size_t(sb) * 144;
+        const uint32_t dm = *reinterpret_cast<const uint32_t *>(blk);
+        const float d = __half2float(__ushort_as_half(uint16_t(dm & 0xffffu))) / kMoeVectorDown, dmin = __half2float(__ushort_as_half(uint16_t(dm >> 16))) / kMoeVectorDown;
+        const uint32_t sw[3] = {*reinterpret_cast<const uint32_t *>(blk + 4), *reinterpret_cast<const uint32_t *>(blk + 8),
+                                *reinterpret_cast<const uint32_t *>(blk + 12)};
+        float sc, mn;
+        q4k_scale_min(sw, sub, sc, mn);
+        const uint2 qs = *reinterpret_cast<const uint2 *>(blk + 16 + 32 * (sub >> 1) + t0);
+        float qx = 0.0f;
+        const uint32_t n0 = (qs.x >> shift) & 0x0F0F0F0Fu, n1 = (qs.y >> shift) & 0x0F0F0F0Fu;  // the lane's eight codes, a byte each
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          // the code as a float without a conversion instruction (quarter rate): 2^23 + q in the mantissa, minus 2^23
+          const float q = __uint_as_float(0x4B000000u | __byte_perm(j < 4 ? n0 : n1, 0, 0x4440 + (j & 3))) - 8388608.0f;
+          qx = fmaf(q, xs[j], qx);
+        }
+        acc[m][c] = fmaf(d * sc, qx, acc[m][c]);
+        acc[m][c] = fmaf(-dmin * mn, xsum, acc[m][c]);
+      }
+  }
+#pragma unroll
+  for (int m = 0; m < NM; ++m)
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int o = 16; o; o >>= 1) acc[m][c] += __shfl_xor_sync(0xffffffffu, acc[m][c], o);
+}
+
+// PAIR: gate and up of the route's expert over the row's input -> intermediate. Otherwise: down over the route's
+// intermediate -> y. grid (rows * routes, column blocks).
+template <bool PAIR> __global__ void __launch_bounds__(kMoeThreads) moe_expert_kernel(const MoeParams p) {
+  constexpr int kMoeColsPerWarp = PAIR ? kMoeColsPair : kMoeColsDown;
+  extern __shared__ float xrow[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const SbMoeExpertArgs &a = p.a;
+  const uint32_t route = blockIdx.x, row = route / a.routes, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t k = PAIR ? a.hidden : a.inter, n = PAIR ? a.inter : a.hidden;
+  const uint32_t expert = min(a.selected[route], a.experts_total - 1);
+  const uint16_t *src = PAIR ? static_cast<const uint16_t *>(a.input) + size_t(row) * a.hidden : p.intermediate + size_t(route) * a.inter;
+  for (uint32_t i = tid; i < k; i += kMoeThreads) xrow[i] = bf16_bits_to_float(src[i]) * kMoeVectorDown;
+  __syncthreads();
+  const size_t row_bytes = size_t(k / 256) * 144;
+  const uint8_t *w0 = static_cast<const uint8_t *>(PAIR ? a.gate : a.down) + size_t(expert) * n * row_bytes;
+  const uint8_t *w1 = PAIR ? static_cast<const uint8_t *>(a.up) + size_t(expert) * n * row_bytes : nullptr;
+  const uint32_t c0 = (blockIdx.y * kMoeWarps + warp) * kMoeColsPerWarp;
+  if (c0 >= n) return;  // n is a multiple of 256, so a warp's columns are inside or outside together
+  if (PAIR) {
+    const uint8_t *const rows[2] = {w0 + size_t(c0) * row_bytes, w1 + size_t(c0) * row_bytes};
+    float acc[2][kMoeColsPerWarp];
+    q4k_rows_dot<2, kMoeColsPerWarp>(rows, row_bytes, xrow, k, lane, acc);
+    if (lane < kMoeColsPerWarp) {
+      float g = 0.0f, u = 0.0f;
+#pragma unroll
+      for (int c = 0; c < kMoeColsPerWarp; ++c)
+        if (lane == uint32_t(c)) g = acc[0][c], u = acc[1][c];
+      p.intermediate[size_t(route) * a.inter + c0 + lane] = float_to_bf16_bits(round_bf16(u) * silu_f(round_bf16(g)));
+    }
+  } else {
+    const uint8_t *const rows[1] = {w0 + size_t(c0) * row_bytes};
+    float acc[1][kMoeColsPerWarp];
+    q4k_rows_dot<1, kMoeColsPerWarp>(rows, row_bytes, xrow, k, lane, acc);
+    if (lane < kMoeColsPerWarp) {
+      float v = 0.0f;
+#pragma unroll
+      for (int c = 0; c < kMoeColsPerWarp; ++c)
+        if (lane == uint32_t(c)) v = acc[0][c];
+      p.y[size_t(route) * a.hidden + c0 + lane] = float_to_bf16_bits(v);
+    }
+  }
+}
+
 // out = bf16(residual + sum over the row's routes in slot order of weight * float(y)).
 __global__ void __launch_bounds__(256) moe_combine_kernel(const MoeParams p) {
   pdl_launch_dependents();
@@ -576,6 +690,16 @@ extern "C" int sb_moe_experts_partial(void *stream, const SbMoeExpertArgs *a, ui
   return moe_experts_grouped(as_stream(stream), a, &share);
 }
 
+// Blocks that take a matrix-vector product a route: experts of up to 1024 x 512 and some 4.7 M weights a matrix over all routes.
+// 3, 9 and 18 routes of 1024 x 256: 16.0, 16.7 and 17.6 us against 19.2, 19.6 and 20.0 by groups, 27 routes 21.3 against 22.6, 36
+// routes 25.4 against 23.8; of 1024 x 512 3 and 6 routes 18.0 and 19.0 against 20.6 and 20.5, 10 routes 25.8 against 21.1; wider
+// experts are even at 3 routes (1536 x 512: 22.2 against 22.5) and behind from there. The difference at the small end is two launches.
+constexpr uint32_t kMoeVectorHidden = 1024, kMoeVectorInter = 512;
+constexpr uint64_t kMoeVectorWeights = 18ull * 1024 * 256;
+static bool moe_vector_block(const SbMoeExpertArgs &a) {
+  return a.hidden <= kMoeVectorHidden && a.inter <= kMoeVectorInter && uint64_t(a.rows) * a.routes * a.hidden * a.inter <= kMoeVectorWeights;
+}
+
 extern "C" int sb_moe_experts(void *stream, const SbMoeExpertArgs *a) {
   SB_NEED_DEVICE();
   const int valid = moe_check(a, "sb_moe_experts");
@@ -594,7 +718,15 @@ extern "C" int sb_moe_experts(void *stream, const SbMoeExpertArgs *a) {
                     reinterpret_cast<float *>(base + l.act_scale)};
   cudaStream_t s = as_stream(stream);
   const uint32_t routes = a->rows * a->routes, resident = uint32_t(ctx().sm_count) * 2;
-  int st = launch_moe(moe_few_prepare_kernel, dim3(a->rows + 1), dim3(kMoeThreads), 0, s, p);
+  int st;
+  if (moe_vector_block(*a)) {
+    constexpr uint32_t kPairBlock = kMoeWarps * kMoeColsPair, kDownBlock = kMoeWarps * kMoeColsDown;
+    st = launch_moe(moe_expert_kernel<true>, dim3(routes, (a->inter + kPairBlock - 1) / kPairBlock), dim3(kMoeThreads), size_t(a->hidden) * 4, s, p);
+    if (st == SB_OK) st = launch_moe(moe_expert_kernel<false>, dim3(routes, (a->hidden + kDownBlock - 1) / kDownBlock), dim3(kMoeThreads), size_t(a->inter) * 4, s, p);
+    if (st != SB_OK) return st;
+    return launch_moe(moe_combine_kernel, dim3((a->hidden + 255) / 256, a->rows), dim3(256), 0, s, p);
+  }
+  st = launch_moe(moe_few_prepare_kernel, dim3(a->rows + 1), dim3(kMoeThreads), 0, s, p);
   if (st == SB_OK) st = launch_moe(moe_few_kernel<true>, dim3(resident), dim3(kMoeThreads), 0, s, p);
   if (st == SB_OK) st = launch_moe(moe_few_convert_kernel, dim3(routes), dim3(std::min(uint32_t(kMoeThreads), a->inter / 8)), 0, s, p);
   if (st == SB_OK) st = launch_moe(moe_few_kernel<false>, dim3(resident), dim3(kMoeThreads), 0, s, p);

@@ -14,12 +14,18 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("rows,routes,experts,H,I,choice,offset", [
-    (1, 1, 1, 256, 256, "one", 0),
-    (16, 1, 3, 512, 256, "one", 0),         # sixteen routes of one expert: two full groups
+    (1, 1, 1, 256, 256, "one", 0),          # (experts of up to 1024 x 512 and few routes: a matrix-vector product a route)
+    (16, 1, 3, 512, 256, "one", 0),
+    (9, 2, 4, 1024, 256, "spread", 2),      # the most weights of such a block
+    (1, 1, 1, 1280, 256, "one", 0),
+    (16, 1, 3, 1280, 256, "one", 0),        # sixteen routes of one expert: two full groups
+    (10, 2, 4, 1024, 256, "spread", 2),     # one route too many for it
     (9, 2, 4, 256, 768, "one", 2),          # nine and nine: a group of eight and one of one
     (16, 32, 40, 512, 512, "spread", 0),    # the most routes
     (5, 7, 300, 768, 256, "spread", 6),
     (3, 4, 6, 512, 256, "past", 0),         # an id past the experts reads the last one, as ever
+    (3, 4, 6, 1280, 256, "past", 0),
+    (2, 3, 5, 256, 2304, "spread", 0),      # an intermediate row of more than one round of its conversion
 ])
 def test_few_rows_experts(rows, routes, experts, H, I, choice, offset):
     lib, l, o = _setup()

@@ -178,6 +178,18 @@ def test_attention_long_context_32k(kernel):
     assert cos > 0.9995 and np.abs(got - want64).max() < 0.02
 
 
+def check_gdn_hidden(got, want):
+    """Rows of a Gated-DeltaNet layer (bf16 bits) against the oracle's, every value and every row's every head. What may differ: q, k, v
+    by a bf16 unit where the last bit of a convolution flips (2^-8 of one of 128 terms of an inner product, a handful of them),
+    the recurrent value by the unit of its own rounding, the result by two more (2^-9 each). A head's values share the error of its
+    inner products, so a value's own is held to its units and 2^-5 of the head's size times its gate's, at most some eight times the mean."""
+    g, w = (ol.bf2f(a).astype(np.float64).reshape(a.shape[0], -1, 128) for a in (got, want))
+    assert np.isfinite(g).all()
+    size = np.sqrt((w * w).mean(axis=-1, keepdims=True))
+    assert (np.abs(g - w) <= 4 * ulp_bf16(w) + 2.0 ** -5 * size).all()
+    assert (np.sqrt(((g - w) ** 2).mean(axis=-1, keepdims=True)) <= 2.0 ** -7 * size).all()
+
+
 def gdn_case(lib, l, o, *, key_heads, value_heads, rows, pending_rows, tiled, seed, fused_gates=0, tree=None, pending_path=0):
     """fused_gates = k > 0: b and a are projections of a bf16 input [16, k] by fp32 rows [2 * value_heads, k]; the
     kernel computes them itself (gate_weight / gate_input) and the oracle gets what sb_linear_f32 gives for them."""
@@ -264,6 +276,7 @@ def test_gdn_verify_within_reference_gates(cfg):
     g, w = ol.bf2f(got["hidden"][:rows]).astype(np.float64), ol.bf2f(want["hidden"][:rows]).astype(np.float64)
     bad = np.abs(g - w) > 3 * ulp_bf16(w) + 2e-3 * np.abs(w).mean()
     assert bad.mean() <= 0.01
+    check_gdn_hidden(got["hidden"][:rows], want["hidden"][:rows])
 
 
 def _tree_rows(parent):
@@ -295,6 +308,7 @@ def test_gdn_tree_paths_within_reference_gates(cfg):
     g, w = ol.bf2f(got["hidden"][:rows]).astype(np.float64), ol.bf2f(want["hidden"][:rows]).astype(np.float64)
     bad = np.abs(g - w) > 3 * ulp_bf16(w) + 2e-3 * np.abs(w).mean()
     assert bad.mean() <= 0.01
+    check_gdn_hidden(got["hidden"][:rows], want["hidden"][:rows])
     # every row on its own: a branch's rows differ from what the chain order would give
     for r in range(rows):
         gr, wr = g[r], w[r]
@@ -399,6 +413,7 @@ def test_gdn_fold_call_then_step_on_the_swapped_cells():
     assert np.abs(two["state"] - st2).max() <= 1e-4 * np.abs(st2).max()
     g, w = ol.bf2f(two["hidden"]).astype(np.float64), ol.bf2f(hid2).astype(np.float64)
     assert (np.abs(g - w) > 3 * ulp_bf16(w) + 2e-3 * np.abs(w).mean()).mean() <= 0.01
+    check_gdn_hidden(two["hidden"], hid2)
     assert np.abs(g).max() > 0
     # and fold-then-step is the one-launch step, bit for bit
     for n in ("cs", "state", "hidden", "k"):

@@ -711,12 +711,12 @@ static int gdn_validate(const SbGdnArgs *a, const char *who) {
 }
 }  // namespace sb
 
-static int gdn_launch(void *stream, const SbGdnArgs *a, bool pdl) {
+static int gdn_launch(void *stream, const SbGdnArgs *a, bool pdl, int device) {
   const GdnParams p{*a};
   const bool tree = needs_tree_kernel(*a), several = a->lanes > 1;
   const auto kernel = several ? (tree ? gdn_kernel<true, 4> : gdn_kernel<false, 4>) : (tree ? gdn_kernel<true, 2> : gdn_kernel<false, 2>);
   static std::atomic<uint64_t> allowed[4];
-  const int st = allow_smem(reinterpret_cast<const void *>(kernel), sizeof(GdnShared), allowed[2 * several + tree]);
+  const int st = allow_smem(reinterpret_cast<const void *>(kernel), sizeof(GdnShared), allowed[2 * several + tree], device);
   if (st != SB_OK) return st;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kGdnSplit, a->value_heads, std::max(1u, a->lanes));
@@ -735,7 +735,7 @@ static int gdn_launch(void *stream, const SbGdnArgs *a, bool pdl) {
 extern "C" int sb_gdn_verify(void *stream, const SbGdnArgs *a) {
   SB_NEED_DEVICE();
   const int valid = gdn_validate(a, "sb_gdn_verify");
-  return valid != SB_OK ? valid : gdn_launch(stream, a, ctx().pdl);
+  return valid != SB_OK ? valid : gdn_launch(stream, a, ctx().pdl, ctx().device);
 }
 
 extern "C" int sb_gdn_verify_static(void *stream, const SbGdnArgs *a) {
@@ -744,5 +744,5 @@ extern "C" int sb_gdn_verify_static(void *stream, const SbGdnArgs *a) {
              kStaticMaxValueHeads);
   SB_REQUIRE(a->lanes <= 1, "sb_gdn_verify_static: one lane a call");
   const int valid = gdn_validate(a, "sb_gdn_verify_static");
-  return valid != SB_OK ? valid : gdn_launch(stream, a, false);
+  return valid != SB_OK ? valid : gdn_launch(stream, a, false, -1);  // (no context)
 }

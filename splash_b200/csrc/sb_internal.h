@@ -62,11 +62,11 @@ enum : uint32_t {
   SB_DEV_CONTRACT = 2       // a kernel met arguments outside its contract and returned early
 };
 
-// Lets `kernel` have `bytes` of dynamic shared memory on the current device; the attribute stays with the function, so it is set
-// at the kernel's first launch on a device only (`done`: a bit a device, the kernel's own).
-inline int allow_smem(const void *kernel, size_t bytes, std::atomic<uint64_t> &done) {
-  int device = 0;
-  SB_CUDA(cudaGetDevice(&device));
+// Lets `kernel` have `bytes` of dynamic shared memory on a device (the context's; below 0: the current one, asked for at every call);
+// the attribute stays with the function, so it is set at the kernel's first launch on a device only (`done`: a bit a device, the
+// kernel's own).
+inline int allow_smem(const void *kernel, size_t bytes, std::atomic<uint64_t> &done, int device) {
+  if (device < 0) SB_CUDA(cudaGetDevice(&device));
   const uint64_t bit = uint64_t(1) << (device & 63);
   if (done.load(std::memory_order_acquire) & bit) return SB_OK;
   SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));

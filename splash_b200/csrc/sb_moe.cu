@@ -637,7 +637,7 @@ static int moe_experts_grouped(cudaStream_t s, const SbMoeExpertArgs *a, const M
   {
     cudaLaunchConfig_t cfg = {};
     static std::atomic<uint64_t> allowed;
-    const int st = allow_smem(reinterpret_cast<const void *>(moe_group_kernel), kMoeMaxRoutes * sizeof(uint16_t), allowed);
+    const int st = allow_smem(reinterpret_cast<const void *>(moe_group_kernel), kMoeMaxRoutes * sizeof(uint16_t), allowed, ctx().device);
     if (st != SB_OK) return st;
     cfg.gridDim = dim3(1), cfg.blockDim = dim3(kMoeGroupThreads), cfg.dynamicSmemBytes = n * sizeof(uint16_t), cfg.stream = s;
     cudaLaunchAttribute attr[1];

@@ -793,7 +793,7 @@ template <class A> static int launch_selection(void (*cluster)(A), void (*polici
   if (clusters) {
     static std::atomic<uint64_t> allowed[2];  // (a pair a kind of arguments, that is, one a kernel)
     if (s.lane_policies) cluster = policies;
-    const int st = allow_smem(reinterpret_cast<const void *>(cluster), select_smem_bytes(kSelectVocab), allowed[s.lane_policies ? 1 : 0]);
+    const int st = allow_smem(reinterpret_cast<const void *>(cluster), select_smem_bytes(kSelectVocab), allowed[s.lane_policies ? 1 : 0], ctx().device);
     if (st != SB_OK) return st;
   }
   SB_CUDA(cudaLaunchKernelEx(&cfg, clusters ? cluster : block, args));

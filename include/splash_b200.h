@@ -630,8 +630,8 @@ SB_API int sb_moe_route(void *stream, const SbMoeRouteArgs *args);
  *   out = bf16(residual + sum over the row's routes in slot order of weight * float(y)).
  * Replaces, in that regime, the expert passes and the combine of MoE::addRouted (runtime/ops/MoE.cpp:122-187,260-270;
  * runtime/metal/kernels/common/moe_gguf_expert_tile.h:33-84, runtime/metal/kernels/shared/moe_gguf.metal:94-160,
- * runtime/metal/kernels/shared/moe.metal:367-392). Routes are grouped by expert: eight a group up to 16 rows, per-expert
- * tiles of 64 rows beyond.
+ * runtime/metal/kernels/shared/moe.metal:367-392). Routes are grouped by expert: eight a group up to 16 rows (a few routes of
+ * small experts take a matrix-vector product each), per-expert tiles of 64 rows beyond.
  * gate, up: native Q4_K rows [experts_total][inter][hidden]; down: [experts_total][hidden][inter]; the shared expert,
  * if routed, is expert index `experts` of the same tensors (experts_total counts it). */
 typedef struct SbMoeExpertArgs {

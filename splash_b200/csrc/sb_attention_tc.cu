@@ -18,12 +18,10 @@
 //             by more than 8 (p <= 256 stays far inside fp16); then the thread rescales its row of O in tensor
 //             memory once the previous chunk's P V has completed. The merge weighs splits by their own m.
 //
-// The ends of the kernel, one layer of the 27B shape at 32K with the store of its rows: 60.9 -> 53.6 us with Q turned through shared memory (a thread reading
-// its own row from memory made each load touch 32 lines: 4.9 k cycles) and the partials laid out with the rows next to each
-// other, so a split's stores and the merge's loads are up to 512 consecutive bytes (8.7 k and 12 k cycles before), read once. The loop (4.5 k
-// cycles a chunk) waits for the tensor pipe and tensor memory in turn; tried and slower: the copies issued by a warp of their own
-// (59-61 us), K and V handed over and given back separately (61 us: softmax's tensor-memory accesses take twice as long while
-// MMAs run), waits that sleep between polls (57-58 us).
+//   ends      Q is turned through shared memory (a thread reading its own row from memory makes each load touch 32 lines), and the
+//             partials lie with the rows next to each other, so that a split's stores and the merge's loads are up to 512 consecutive bytes,
+//             read once: one layer of the 27B shape at 32K, with the store of its rows, 55.3 us (63.5 without either). What bounds the
+//             kernel is the loop, some 4.5 k cycles a chunk, which waits for the tensor pipe and tensor memory in turn.
 //
 // Tensor-memory columns: Q [0, D/2), S / P double buffer 2 x 64, O D columns: 512 at D = 256.
 #include <algorithm>
@@ -119,7 +117,6 @@ __global__ void __launch_bounds__(kAtThreads, 1) attention_tc_kernel(const AttnP
       constexpr uint32_t kPitch = 128 * 2;  // (16-byte units of a row exchanged by its low bits: no two of eight lanes share a bank either way)
       static_assert(2 * 32 * kPitch <= L::kConvBytes, "two warps' rows in a buffer");
       uint8_t *turn = smem + (warp < 2 ? L::kK : L::kV) + L::kConvBytes + (warp & 1) * 32 * kPitch;
-      
       uint4 raw[D / 128][16];  // every load in flight at once
 #pragma unroll
       for (int i = 0; i < 16; ++i) {

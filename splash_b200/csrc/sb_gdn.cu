@@ -14,20 +14,18 @@
 //            (3) fold the pending rows into the state -> committed state stored; (4) the rows' outputs from the
 //            committed state; (5) RMS norm over the 128 value dimensions, gate by silu(z), the hidden rows; (6) this step's tape
 //
-// The delta rule without its serial chain. A row's step S' = d S + u k^T, u = beta (v - d S k) touches the whole state, and 22
-// of them (6 folded, 16 scanned) one after the other, each a reduction across lanes, took most of the kernel (23.4 us a call
-// of one lane, 106 us of eight, where moving the state takes 1 and 8). The state after the block is never stored, so it is
-// never formed: with S the committed state, P(t) a row's path from the anchor and G(t, j) the product of the decays on it
-// after row j (D_t: of all of them),
+// The delta rule without its serial chain. A row's step S' = d S + u k^T, u = beta (v - d S k) touches the whole state, one row after
+// the other. The state after the block is never stored, so it is never formed: with S the committed state, P(t) a row's path from
+// the anchor and G(t, j) the product of the decays on it after row j (D_t: of all of them),
 //   u_t = beta_t (v_t - D_t (S k_t) - sum over j in P(t), j != t, of G(t, j) (k_j . k_t) u_j)
 //   o_t = D_t (S q_t) + sum over j in P(t) of G(t, j) (k_j . q_t) u_j
 // that is: the 16 x 128 by 128 products S k_t and S q_t, all rows at once from registers; the rows' inner products; and a
 // triangular system of 16 unknowns per state row, one thread each. Chains and trees are the same formulas. The fold is the same
-// system over the pending rows, then one update of rank `pending`: S = D S + sum_t G(last, t) u_t k_t^T. One layer of the 27B
-// shape takes 13.6 us instead of 23.4, eight lanes 73 instead of 106 (the kernel alone, in a graph); the folded state's error
-// against 64 bits stays at 6e-8, and that of the rows' outputs at their bf16. What bounds it now is the prologue's latency
-// (dependent loads, the gate projection), four cluster barriers, and, with many lanes, instruction issue (half of the slots) and the
-// shared-memory port.
+// system over the pending rows, then one update of rank `pending`: S = D S + sum_t G(last, t) u_t k_t^T.
+// What bounds it: the prologue's latency (dependent loads, the gate projection), four cluster barriers, and, with many lanes, instruction
+// issue (half of the slots) and the shared-memory port. One layer of the 27B shape, 16 rows and 6 to fold, graph replay: 13.8 us (23.7
+// with the rows advanced in turn), eight lanes 68 (100), one row and one to fold 10.5 (11.3), eight lanes of those 48.0 (47.7). The
+// folded state's error against 64 bits is 5.6e-8 either way, that of the rows' outputs their bf16.
 //   CTA      256 threads; warp w owns rows 16 (w & 1).. of the CTA's 32 and key columns 32 (w / 2).. , in fp32 registers laid out as
 //            the tensor cores' A operand
 //   rollback the state after the block is never stored: the caller passes how many tape rows were accepted

@@ -148,8 +148,7 @@ __device__ __forceinline__ bool wide_warp_spin(uint64_t *bar, uint32_t parity) {
 // consecutive inputs the order is [0, 2, 1, 3]: the order in which the weight expansion produces its halves.
 // A chain of latencies (the row, its statistics, the row again), so a row has as many threads as fill whole rounds of its chunks,
 // every split's loads are in flight together and the norm's weights are fetched beside the row: 128 rows of 5120 take 5.3 us
-// (7.2 with 256 threads and loads one after the other), with seven splits to add 8.4 (13.2). Tried: eight rows by a cluster of
-// eight CTAs, so that stores are whole lines (10.9 and 25 us).
+// (7.2 with 256 threads and loads one after the other), with seven splits to add 8.4 (13.2).
 constexpr uint32_t kWidePrepMost = 768;
 // Threads for rows of `chunks` chunks: as few rounds as kWidePrepMost allows, evenly filled.
 static uint32_t wide_prep_threads(uint32_t chunks) {
@@ -674,10 +673,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) linear_wide_kernel(const Wide
         if (rs >= kWideRawStages) rs -= kWideRawStages, rphase ^= 1;
         {
           WIDE_T0();
-          // The hand-over between this warp and the MMA thread paces the kernel: its waits never park, and every lane polls for
-          // itself (a MoE block of 512 rows 320.6 -> 306 us, a feed-forward block of 128 rows 104.0 -> 102.2). Finer
-          // hand-overs, so that a buffer's first half is refilled while its second is read, cost more than they hide: 128 rows
-          // gate / up 49.0 -> 56.3 us.
+          // The hand-over between this warp and the MMA thread paces the kernel, so its waits never park.
           if (scount > 0 && !wide_warp_spin(&a_empty[ab], (scount - 1) & 1)) {
             if (lane == 0) wide_expired(p.status, 7);
             ok = false;

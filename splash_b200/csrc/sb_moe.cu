@@ -1,19 +1,18 @@
-// MoE expert passes for the few rows of one lane's verify block (M <= 16 rows, up to 32 routes a row): every route
-// (row, expert) is a matrix-vector product against the expert's native Q4_K rows. Replaces, for that regime, the
-// expert passes of MoE::addRouted (runtime/ops/MoE.cpp:122-187,260-270; kernels moe_gguf_expert_tile of
-// runtime/metal/kernels/common/moe_gguf_expert_tile.h:33-84, the gate/up pass runtime/metal/kernels/shared/moe_gguf.metal:
+// MoE expert passes. Replaces the expert passes of MoE::addRouted (runtime/ops/MoE.cpp:122-187,260-270; kernels moe_gguf_expert_tile
+// of runtime/metal/kernels/common/moe_gguf_expert_tile.h:33-84, the gate/up pass runtime/metal/kernels/shared/moe_gguf.metal:
 // 94-160 and moe_combine, runtime/metal/kernels/shared/moe.metal:367-392):
 //   intermediate = bf16(bf16(up . x) * silu(bf16(gate . x)))     per route
 //   y            = bf16(down . intermediate)                     per route
 //   out          = bf16(residual + sum over the row's routes, in slot order, of weight * float(y))
-// The routes are grouped by expert (up to eight a group, the columns of one MMA), so an expert's weights are read once for all the
-// rows that chose it. A matrix-vector product a route (the first form) spent some 3 instructions a weight and route: 186 us for 16
-// rows of the 35B-A3B shape, 1.0 TB/s. Now a warp takes 16 gate and the 16 up rows (32 down rows) of a group over the whole of K:
-// lane 4 g + t loads rows g and g + 8's sub-blocks 2t, 2t + 1 of every super-block straight into registers (two 16-byte loads a row
-// and a header) and feeds them to mma.sync as exact integers sc q (sb_q4k.cuh) against the group's activations in fp16, exact too
-// (a power of two a row), the block scales on fp32 sums: 76 us for the same 16 rows, 180 MB of experts' weights in some 62 us of two
-// expert passes (2.6 TB/s). What bounds them is the L1: a warp's 16-byte loads touch eight rows each, and the activations come the
-// same way. Tried: the next unit's rows prefetched into the L2 (84 us), three CTAs a SM at 80 registers (78 us).
+// A lane's block (up to 16 rows, up to 32 routes each): the routes are grouped by expert (up to eight a group, the columns of one
+// MMA), so an expert's weights are read once for all the rows that chose it; blocks of small experts take a matrix-vector product a
+// route (moe_vector_block). More rows: the groups are tiles of the many-row projection (below).
+// A warp takes 16 gate and the 16 up rows (32 down rows) of a group over the whole of K: lane 4 g + t loads rows g and g + 8's sub-blocks
+// 2t, 2t + 1 of every super-block straight into registers (two 16-byte loads a row and a header) and feeds them to mma.sync as
+// exact integers sc q (sb_q4k.cuh) against the group's activations in fp16 (a power of two a row), the block scales on fp32 sums.
+// 16 rows of the 35B-A3B shape, routing included, graph replay: 77 us (185 with a product a route), 180 MB of experts' weights in 45 and
+// 24 us of the two passes (ncu, cold: 2.6 TB/s). What bounds them is the L1: a warp's 16-byte loads touch eight rows each, and the
+// activations come the same way.
 #include <algorithm>
 
 #include "sb_internal.h"

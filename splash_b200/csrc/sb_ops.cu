@@ -527,7 +527,9 @@ __device__ __forceinline__ void sample_row(const SbSampleArgs &a, uint32_t r) {
 }
 
 // Whether a greedy lane's rows take a CTA each, eight neighbouring rows a cluster and the lane's other clusters none, in a launch whose
-// lanes have policies of their own (known on the device only): where it has more rows than a greedy launch gives a cluster each.
+// lanes have policies of their own (known on the device only): where it has more rows than a greedy launch gives a cluster each. All
+// lanes greedy, 128 rows of 151,936: 29.9 us against 35.8 with a cluster a row, 512 rows 82 against 147; of 248,320 (one CTA a SM) 59
+// against 79, 146 against 280. Half of the lanes sampled, 512 rows of 151,936: 0.56 ms against 0.71.
 constexpr uint32_t kGreedyClusterRows = 32;
 __device__ __forceinline__ bool alone_in_cluster(const SbSampleArgs &a, uint32_t lane) {
   return a.rows * max(a.lanes, 1u) > kGreedyClusterRows && a.lane_policies[lane].temperature == 0.0f;
@@ -764,8 +766,8 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const SbMoeRouteArgs a) 
 
 // A selection over rows x lanes: the cluster kernel up to its vocabulary (a greedy launch keeps no logits in shared memory), the
 // block kernel above. A greedy row is one short pass, and what counts is how many rows run at once: 37 clusters are resident
-// (two CTAs a SM), so up to 32 greedy rows take clusters (16 rows of 151,936: 15.1 us against 20.8 with a block a row) and more
-// take a block each, all resident together (128 rows: 29.6 us against 38.4; 512 rows: 92 against 133). Sampled rows are the
+// (two CTAs a SM), so up to 32 greedy rows take clusters (16 rows of 151,936: 11.2 us against 17.2 with a block a row) and more
+// take a block each, all resident together (128 rows: 22.4 us against 35.8; 512 rows: 91 against 147). Sampled rows are the
 // other way round (128 rows without filters: 122 us against 182; 512 rows: 423 against 548) until the vocabulary leaves room
 // for one CTA a SM only (above some 160,000 ids): without filters 128 rows of 232,001 take 220 us against 259, 512 rows 804
 // against 800, so from 256 such rows on a row is a block's; with filters clusters win at every count (512 rows: 2.1 ms

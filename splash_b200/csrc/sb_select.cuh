@@ -11,11 +11,12 @@
 //     approximate masses) names the bin the end lies in, and the bin's tokens, gathered by CTA 0, name the key;
 //   - masses that decide anything are still the sums in the fixed order: a key found from approximate masses is taken only if
 //     the exact masses at it and above it say so (the exact mass only grows with the set, every weight being >= 0, so the
-//     key with that property is the one the bit-by-bit search ends at). Otherwise, or when a bin holds more tokens than the
-//     list, or a row's largest logit or the temperature makes a weight no number, the search walks the bits as before.
-// The 128 rows above take 275 us, 16 such rows 71 us (5.68 ms), 16 rows without filters 37 us (166). What is left is the passes
-// themselves (a few instructions for each of 152 k tokens a pass, 37 rows resident at a time) and the ordered sums.
-// The tokens and ends selected are the same, bit for bit, as those of one block a row walking the bits.
+//     key with that property is the one a bit-by-bit search ends at). Where the nucleus's end lies among so many tokens that the
+//     list does not hold them, or that one weighs less than the roundings, the tokens around it are sorted and searched by exact
+//     masses. Otherwise, or when a row's largest logit or the temperature makes a weight no number, the search walks the bits.
+// The 128 rows above take 268 us, 16 such rows 69 us (5.67 ms), 16 rows without filters 34 us (158), 128 rows at top-p 0.95 and
+// temperature 1 without top-k 1.2 ms (3.1). What is left is the passes themselves (a few instructions for each of 152 k tokens a
+// pass, 37 rows resident at a time) and the ordered sums.
 #pragma once
 
 namespace sb {

@@ -481,8 +481,8 @@ template <bool TP> __global__ void __launch_bounds__(kPrepThreads) prepare_kerne
     }
   }
   const int e = row_exponent(mx);
-  const float down = ldexpf(1.0f, -e);
-  if (tid == 0 && rank == 0) reinterpret_cast<float *>(p.out)[tok] = ldexpf(1.0f, e);
+  const float down = power_of_two(-e);
+  if (tid == 0 && rank == 0) reinterpret_cast<float *>(p.out)[tok] = power_of_two(e);
   const uint32_t h = tok >> 3, g = tok & 7;
 #pragma unroll
   for (int i = 0; i < kPrepMaxChunks; ++i) {

@@ -286,8 +286,8 @@ __global__ void __launch_bounds__(kWidePrepMost) wide_prepare_kernel(const WideP
     mx = mx * inv * 1.0625f;  // (x inv) w against x w inv and the rounding to bf16: well inside 6 %
   }
   const int e = row_exponent(mx);
-  const float down = ldexpf(1.0f, -e);
-  if (tid == 0) reinterpret_cast<float *>(p.out)[tok] = live ? ldexpf(1.0f, e) : 0.0f;
+  const float down = power_of_two(-e);
+  if (tid == 0) reinterpret_cast<float *>(p.out)[tok] = live ? power_of_two(e) : 0.0f;
   auto convert = [&](uint32_t c, const uint4 raw) {
     uint4 h = make_uint4(0, 0, 0, 0);
     if (live) {
@@ -357,8 +357,8 @@ __global__ void __launch_bounds__(kWideSlotThreads) wide_prepare_slots_kernel(co
 #pragma unroll
   for (int w = 0; w < kWideSlotWarps; ++w) mx = fmaxf(mx, warp_s[w][tid & 7]);
   const int e = row_exponent(mx);
-  const float down = ldexpf(1.0f, -e);
-  if (tid < kWideSlotRows) p.scales[slot] = live ? ldexpf(1.0f, e) : 0.0f;
+  const float down = power_of_two(-e);
+  if (tid < kWideSlotRows) p.scales[slot] = live ? power_of_two(e) : 0.0f;
   auto convert = [&](uint32_t c, const uint4 raw) {
     uint4 h = make_uint4(0, 0, 0, 0);
     if (live) {

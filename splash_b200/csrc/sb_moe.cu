@@ -90,8 +90,8 @@ __device__ __forceinline__ void moe_convert_row(const uint16_t *src, uint32_t k,
   __syncthreads();
   for (uint32_t w = 0; w < blockDim.x / 32; ++w) mx = fmaxf(mx, scratch[w]);
   const int e = row_exponent(mx);
-  const float down = ldexpf(1.0f, -e);
-  if (tid == 0) *scale = ldexpf(1.0f, e);
+  const float down = power_of_two(-e);
+  if (tid == 0) *scale = power_of_two(e);
 #pragma unroll
   for (int i = 0; i < kMost; ++i) {
     const uint32_t c = tid + i * blockDim.x;

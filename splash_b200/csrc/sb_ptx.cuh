@@ -179,13 +179,11 @@ __device__ __forceinline__ float round_bf16(float f) { return __bfloat162float(_
 // 2^10. Never below -126, so that 2^-e stays finite for rows near bf16's smallest magnitudes (their scaled values are then
 // smaller, and still exact: bf16 reaches down to 2^-133). A row with an infinity keeps its values.
 __device__ __forceinline__ int row_exponent(float mx) {
-  int e = 0;
-  if (mx > 0.0f && mx < INFINITY) {
-    (void)frexpf(mx, &e);  // mx = f * 2^e with f in [0.5, 1)
-    e = max(e - 10, -126);
-  }
-  return e;
+  const uint32_t bits = __float_as_uint(mx);  // (never negative; mx = f * 2^(bits >> 23 - 126) with f in [0.5, 1) unless subnormal)
+  return bits > 0 && bits < 0x7f800000u ? max(int(bits >> 23) - 126 - 10, -126) : 0;
 }
+// 2^e for e in -126 .. 127.
+__device__ __forceinline__ float power_of_two(int e) { return __uint_as_float(uint32_t(127 + e) << 23); }
 
 // e^-x as exp2(-x log2 e): the form every activation of the verify step uses.
 // The quotient is the approximate one (reciprocal and multiply, 2 ulp): every result is rounded to bf16 next.
